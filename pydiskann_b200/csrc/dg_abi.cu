@@ -119,6 +119,8 @@ DgStatus dg_index_create(const DgIndexDesc *desc, DgIndex **out) {
     dg_index_destroy(idx);
     return st;
   };
+  if (cudaDeviceGetAttribute(&idx->sms, cudaDevAttrMultiProcessorCount, idx->device) != cudaSuccess)
+    return bail(fail(DG_EDEVICE, "device attributes"));
   if (cudaStreamCreateWithFlags(&idx->stream, cudaStreamNonBlocking) != cudaSuccess)
     return bail(fail(DG_EDEVICE, "stream creation failed"));
   if ((s = dev_alloc(idx, (void **)&idx->vec, idx->n * idx->dpad * 4)) != DG_OK) return bail(s);
@@ -489,6 +491,75 @@ static void index_state(const DgIndex *idx, SearchArgs &a) {
   a.code_limit = idx->code_limit && idx->code_limit < idx->n ? idx->code_limit : idx->n;
 }
 
+// Bytes of one row of a traversal.
+static uint32_t traversal_row_bytes(const DgIndex *idx, int trav) {
+  switch (trav) {
+    case TRAV_F32: return idx->dpad * 4;
+    case TRAV_BF16: return idx->dpad * 2;
+    case TRAV_FP8: return idx->dpad;
+    default: return idx->code_stride;
+  }
+}
+
+// The kernel of one search of nq queries and its shared-memory layout: a CTA of
+// 8, 4, 2 or 1 warps per query, or the register-list kernel (one warp per
+// query, beams up to 64 without a filter).  Every result is the same.
+//
+// More warps shorten a query's chain of expansions, fewer leave more queries
+// in flight, so a search takes the widest CTA with which every query is
+// resident at once: 2 CTAs of 8 warps, 5 of 4, 10 of 2 or 20 of 1 per SM.
+// Measured (us per call, 300k x 128, 8 / 4 / 2 / 1 warps): FP32, beam 100, 256
+// queries 785 / 823 / 951 / 1221, 740 queries 1445 / 958 / 1063 / 1332, 1200
+// queries 2168 / 1251 / 1095 / 1344, 6000 queries 9008 / 4413 / 3003 / 2459;
+// BF16 with filters, 740 queries 5261 / 3041 / 2765 / 3073 (an expansion finds
+// few new neighbours there: 4 warps never win), 3000 queries - / 8931 / 5221 /
+// 4043.  Short rows skip the 2-warp step (int8, beam 100: 1470 queries 1049 us
+// with 2 warps, 1500 queries 837 with 1).  Where a query's state leaves room
+// for few queries per SM, warps are added instead: PQ tables of 16 KB (8
+// queries), 5000 queries 7365 / 4028 / 3648 / 4430 (then 3270 with 2 warps and
+// 32-code batches); 768-d int8 cosine (11 queries), 4000 queries 12499 / 7209 /
+// 7892 / 12397.
+// The register-list kernel keeps full batches, and small ones whose rows are
+// short (int8 128-d, beam 40: 231 against 247 us for 16 queries, 344 against
+// 472 for 740; FP32 128-d: 369 against 255 for 16, 817 against 637 for 1200,
+// 833 against 822 for 2000; 768-d int8: 912 against 327 for 16).
+struct SearchPlan {
+  WarpLayout Ly;
+  uint32_t cta;         // warps of the CTA a query takes, 0 = register-list kernel
+  bool tc;              // BF16 rows take tensor-core distances
+  uint32_t limit_smem;  // what decides whether the search is accepted, whichever kernel runs
+};
+static SearchPlan plan_search(const DgIndex *idx, int trav, int lcap, bool filt, uint64_t need, uint32_t search_k,
+                              bool reranked, uint32_t hbits, uint32_t wpb, uint32_t nq) {
+  SearchPlan P;
+  const bool decode = (trav == TRAV_RABITQ || trav == TRAV_INT8) && met_kind(idx->metric) != MET_L2;
+  const WarpLayout reg = warp_layout(trav, lcap, filt, hbits, idx->dpad, idx->pq_M, idx->pq_K, idx->rq_padded, decode,
+                                     idx->R, true);
+  P.limit_smem = reg.total * ((wpb == 1 || wpb == 2) ? wpb : 4u);
+  P.tc = lcap == 64 && !filt;
+  // a label-free query of a filtered batch on an index with tombstones may hold
+  // more than the labelled ones (tombstone_config)
+  const uint64_t tneed = idx->tomb && idx->ntomb > 0 ? search_k + std::min<uint64_t>(idx->ntomb, need) : 0;
+  const uint32_t rcap = filt ? search_k : 0, wcap = (uint32_t)std::min<uint64_t>(std::max(need, tneed), 1024);
+  P.Ly = cta_layout(trav, wcap, rcap, reranked ? std::min(search_k, filt ? rcap : wcap) : 0, filt, hbits, idx->dpad,
+                    idx->pq_M, idx->pq_K, idx->rq_padded, decode, idx->R);
+  const uint32_t row = traversal_row_bytes(idx, trav), sms = (uint32_t)idx->sms;
+  const uint32_t room = 227u * 1024u / (P.Ly.total + 1024u);  // queries whose state an SM holds
+  // traversals whose lone warp takes 32 candidates at a time (cta_batch)
+  const bool short_rows = trav == TRAV_INT8 || trav == TRAV_FP8 || trav == TRAV_PQ || trav == TRAV_RABITQ ||
+                          ((trav == TRAV_BF16 || trav == TRAV_F16) && lanes_per_row(idx->dpad / 8) != 8);
+  if (nq <= 2 * sms) P.cta = 8;
+  else if (nq <= 5 * sms && !filt) P.cta = 4;
+  else if (nq <= 10 * sms && !(short_rows && room >= 16)) P.cta = 2;
+  else P.cta = room >= 16 ? 1 : room >= 6 ? 2 : 4;
+  if (P.tc) {
+    const bool long_rows = row >= 256 || idx->dpad >= 512;
+    if (!long_rows || nq > (row >= 512 || idx->dpad >= 512 ? 8 : 5) * sms || room == 0) P.cta = 0;
+  }
+  if (P.cta == 0) P.Ly = reg;
+  return P;
+}
+
 // Stack depth a postfix program needs; -1 if it is malformed.
 static int program_depth(const DgFilterOp *ops, uint32_t n, uint64_t pool_len) {
   int sp = 0, mx = 0;
@@ -745,10 +816,6 @@ DgStatus dg_search_batch(DgIndex *idx, const DgSearchParams *p, const float *que
   if (trav == TRAV_F32) lpr = 8;
   else if (trav == TRAV_BF16 || trav == TRAV_F16) lpr = lanes_per_row(idx->dpad / 8);
   else if (trav == TRAV_INT8) lpr = lanes_per_row(idx->code_stride / 16);
-  const WarpLayout Ly = warp_layout(trav, lcap, filt, hbits, idx->dpad, idx->pq_M, idx->pq_K,
-                                    idx->rq_padded,
-                                    (trav == TRAV_RABITQ || trav == TRAV_INT8) && met_kind(idx->metric) != MET_L2,
-                                    idx->R, true);
   auto launch = [&](const SearchArgs &a0, cudaStream_t ss) -> DgStatus {
     LaunchInfo info;
     SearchArgs aa = a0;
@@ -759,14 +826,16 @@ DgStatus dg_search_batch(DgIndex *idx, const DgSearchParams *p, const float *que
       aa.perm = perm + q0;
     }
     DG_CUDA(cudaMemsetAsync(aa.counter, 0, 4, ss));
+    const SearchPlan P = plan_search(idx, trav, lcap, filt, need, search_k, reranked, hbits, sched.wpb, nq);
+    aa.limit_smem = P.limit_smem;
     switch (trav) {
-      case TRAV_F32: return launch_search_f32(aa, Ly, met, lpr, lcap, filt, ss, &info);
-      case TRAV_BF16: return launch_search_bf16(aa, Ly, met, lpr, lcap, filt, ss, &info);
-      case TRAV_F16: return launch_search_f16(aa, Ly, met, lpr, lcap, filt, ss, &info);
-      case TRAV_INT8: return launch_search_int8(aa, Ly, met, lpr, lcap, filt, ss, &info);
-      case TRAV_PQ: return launch_search_pq(aa, Ly, met, lpr, lcap, filt, ss, &info);
-      case TRAV_FP8: return launch_search_fp8(aa, Ly, met, lpr, lcap, filt, ss, &info);
-      default: return launch_search_rabitq(aa, Ly, met, lpr, lcap, filt, ss, &info);
+      case TRAV_F32: return launch_search_f32(aa, P.Ly, met, lpr, P.cta, P.tc, filt, ss, &info);
+      case TRAV_BF16: return launch_search_bf16(aa, P.Ly, met, lpr, P.cta, P.tc, filt, ss, &info);
+      case TRAV_F16: return launch_search_f16(aa, P.Ly, met, lpr, P.cta, P.tc, filt, ss, &info);
+      case TRAV_INT8: return launch_search_int8(aa, P.Ly, met, lpr, P.cta, P.tc, filt, ss, &info);
+      case TRAV_PQ: return launch_search_pq(aa, P.Ly, met, lpr, P.cta, P.tc, filt, ss, &info);
+      case TRAV_FP8: return launch_search_fp8(aa, P.Ly, met, lpr, P.cta, P.tc, filt, ss, &info);
+      default: return launch_search_rabitq(aa, P.Ly, met, lpr, P.cta, P.tc, filt, ss, &info);
     }
   };
   if (chunks > 1) {
@@ -1188,19 +1257,17 @@ extern "C" DgStatus dg_search_batch_static(DgIndex *idx, const DgSearchParams *p
   if (trav == TRAV_F32) lpr = 8;
   else if (trav == TRAV_BF16 || trav == TRAV_F16) lpr = lanes_per_row(idx->dpad / 8);
   else if (trav == TRAV_INT8) lpr = lanes_per_row(idx->code_stride / 16);
-  const WarpLayout Ly = warp_layout(trav, lcap, filt, hbits, idx->dpad, idx->pq_M, idx->pq_K,
-                                    idx->rq_padded,
-                                    (trav == TRAV_RABITQ || trav == TRAV_INT8) && met_kind(idx->metric) != MET_L2,
-                                    idx->R, true);
+  const SearchPlan P = plan_search(idx, trav, lcap, filt, need, search_k, reranked, hbits, 0, nq);
+  a.limit_smem = P.limit_smem;
   LaunchInfo info;
   switch (trav) {
-    case TRAV_F32: s = launch_search_f32(a, Ly, met, lpr, lcap, filt, st, &info); break;
-    case TRAV_BF16: s = launch_search_bf16(a, Ly, met, lpr, lcap, filt, st, &info); break;
-    case TRAV_F16: s = launch_search_f16(a, Ly, met, lpr, lcap, filt, st, &info); break;
-    case TRAV_INT8: s = launch_search_int8(a, Ly, met, lpr, lcap, filt, st, &info); break;
-    case TRAV_PQ: s = launch_search_pq(a, Ly, met, lpr, lcap, filt, st, &info); break;
-    case TRAV_FP8: s = launch_search_fp8(a, Ly, met, lpr, lcap, filt, st, &info); break;
-    default: s = launch_search_rabitq(a, Ly, met, lpr, lcap, filt, st, &info); break;
+    case TRAV_F32: s = launch_search_f32(a, P.Ly, met, lpr, P.cta, P.tc, filt, st, &info); break;
+    case TRAV_BF16: s = launch_search_bf16(a, P.Ly, met, lpr, P.cta, P.tc, filt, st, &info); break;
+    case TRAV_F16: s = launch_search_f16(a, P.Ly, met, lpr, P.cta, P.tc, filt, st, &info); break;
+    case TRAV_INT8: s = launch_search_int8(a, P.Ly, met, lpr, P.cta, P.tc, filt, st, &info); break;
+    case TRAV_PQ: s = launch_search_pq(a, P.Ly, met, lpr, P.cta, P.tc, filt, st, &info); break;
+    case TRAV_FP8: s = launch_search_fp8(a, P.Ly, met, lpr, P.cta, P.tc, filt, st, &info); break;
+    default: s = launch_search_rabitq(a, P.Ly, met, lpr, P.cta, P.tc, filt, st, &info); break;
   }
   if (s != DG_OK) return s;
   // Record the search's completion on a slot event (created with the index,

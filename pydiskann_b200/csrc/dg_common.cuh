@@ -117,42 +117,38 @@ __device__ __forceinline__ uint64_t range_of(uint64_t r, uint64_t n) { return __
 
 // ------------------------------------------------------------------ filter
 // Postfix evaluation of a DgFilterOp program over one label row
-// (Filter::matches, src/filtered.rs:120-135).
+// (Filter::matches, src/filtered.rs:120-135); label(f) is field f < nf.
 constexpr int kFilterStack = 32;
-__device__ __forceinline__ bool filter_eval(const DgFilterOp *prog, uint32_t nops,
-                                            const uint64_t *pool, const uint64_t *labels,
-                                            uint32_t nf) {
+template <typename Label>
+__device__ __forceinline__ bool filter_eval_by(const DgFilterOp *prog, uint32_t nops, const uint64_t *pool,
+                                               uint32_t nf, Label label) {
   if (nops == 0) return true;
   uint32_t stack = 0;  // bit stack
   int sp = 0;
   for (uint32_t i = 0; i < nops; ++i) {
     const DgFilterOp o = prog[i];
     bool v = false;
-    switch (o.op) {
-      case DG_F_TRUE: v = true; break;
-      case DG_F_EQ: v = o.field < nf && labels[o.field] == o.a; break;
-      case DG_F_IN:
-        if (o.field < nf) {
-          const uint64_t x = labels[o.field];
-          for (uint64_t t = 0; t < o.b; ++t)
-            if (pool[o.a + t] == x) { v = true; break; }
-        }
-        break;
-      case DG_F_LT: v = o.field < nf && labels[o.field] < o.a; break;
-      case DG_F_GT: v = o.field < nf && labels[o.field] > o.a; break;
-      case DG_F_RANGE: v = o.field < nf && labels[o.field] >= o.a && labels[o.field] <= o.b; break;
-      case DG_F_AND:
-      case DG_F_OR: {
-        bool acc = o.op == DG_F_AND;
-        for (uint32_t t = 0; t < o.field && sp > 0; ++t) {
-          --sp;
-          bool x = (stack >> sp) & 1u;
-          acc = (o.op == DG_F_AND) ? (acc && x) : (acc || x);
-        }
-        v = acc;
-        break;
+    if (o.op == DG_F_AND || o.op == DG_F_OR) {  // the top o.field bits
+      const int n = min((int)min(o.field, (uint32_t)kFilterStack), sp);
+      sp -= n;
+      const uint32_t all = n >= 32 ? 0xffffffffu : (1u << n) - 1u;
+      const uint32_t bits = sp < 32 ? (stack >> sp) & all : 0u;
+      v = o.op == DG_F_AND ? bits == all : bits != 0u;
+    } else if (o.op == DG_F_TRUE) {
+      v = true;
+    } else if (o.field < nf) {
+      const uint64_t x = label(o.field);
+      if (o.op == DG_F_EQ) {
+        v = x == o.a;
+      } else if (o.op == DG_F_IN) {
+        for (uint64_t t = 0; t < o.b && !v; ++t) v = pool[o.a + t] == x;
+      } else if (o.op == DG_F_LT) {
+        v = x < o.a;
+      } else if (o.op == DG_F_GT) {
+        v = x > o.a;
+      } else if (o.op == DG_F_RANGE) {
+        v = x >= o.a && x <= o.b;
       }
-      default: v = false;
     }
     if (sp < kFilterStack) {
       stack = v ? (stack | (1u << sp)) : (stack & ~(1u << sp));
@@ -160,6 +156,10 @@ __device__ __forceinline__ bool filter_eval(const DgFilterOp *prog, uint32_t nop
     }
   }
   return sp > 0 ? ((stack >> (sp - 1)) & 1u) : true;
+}
+__device__ __forceinline__ bool filter_eval(const DgFilterOp *prog, uint32_t nops, const uint64_t *pool,
+                                            const uint64_t *labels, uint32_t nf) {
+  return filter_eval_by(prog, nops, pool, nf, [&](uint32_t f) { return labels[f]; });
 }
 
 }  // namespace dg

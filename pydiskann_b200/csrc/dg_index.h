@@ -10,6 +10,7 @@
 
 struct DgIndex {
   int device = 0;
+  int sms = 148;  // SMs of the device
   uint64_t n = 0;
   uint32_t d = 0, dpad = 0, R = 0, medoid = 0;
   int32_t metric = DG_L2SQ;

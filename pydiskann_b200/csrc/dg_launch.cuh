@@ -4,7 +4,7 @@
 #include <mutex>
 #include <unordered_map>
 
-#include "dg_search_kernel.cuh"
+#include "dg_search_cta.cuh"
 
 namespace dg {
 
@@ -14,9 +14,8 @@ struct LaunchInfo {
   uint32_t smem = 0;
 };
 
-// Launch geometry: 4 warps per block (or the schedule's 2 or 1), as many
-// resident blocks as shared memory and registers allow on every SM, never more
-// warps than queries.
+// Launch geometry: as many resident CTAs as shared memory and registers allow
+// on every SM, never more than the queries need.
 // Resident blocks per SM of (device, kernel, shared-memory size), and the
 // largest dynamic shared memory already granted to (device, kernel): the
 // attribute and occupancy queries run once, not on every launch (a serving
@@ -32,11 +31,11 @@ inline LaunchGeometry &launch_geometry() {
   return g;
 }
 
+// `queries` per CTA of `warps` warps, Ly.total bytes of shared memory each.
 template <typename K>
-DgStatus launch_persistent(K kernel, const SearchArgs &a, const WarpLayout &Ly, cudaStream_t st,
-                           LaunchInfo *info) {
-  const uint32_t wpb = (a.wpb == 1 || a.wpb == 2) ? a.wpb : 4u;  // warps per CTA
-  const uint32_t smem = Ly.total * wpb;
+DgStatus launch_persistent(K kernel, const SearchArgs &a, const WarpLayout &Ly, uint32_t warps, uint32_t queries,
+                           cudaStream_t st, LaunchInfo *info) {
+  const uint32_t smem = Ly.total * queries;
   int dev = 0;
   DG_CUDA(cudaGetDevice(&dev));
   LaunchGeometry &G = launch_geometry();
@@ -55,7 +54,7 @@ DgStatus launch_persistent(K kernel, const SearchArgs &a, const WarpLayout &Ly, 
       s_it = G.sms.emplace(dkey, m).first;
     }
     sms = s_it->second;
-    if (smem > (uint32_t)G.optin[dkey])
+    if (std::max(smem, a.limit_smem) > (uint32_t)G.optin[dkey])
       return fail(DG_ENOTSUP, "search state does not fit in shared memory (beam/quantizer too large)");
     int &gr = G.granted[key];
     if ((int)smem > gr) {
@@ -63,11 +62,11 @@ DgStatus launch_persistent(K kernel, const SearchArgs &a, const WarpLayout &Ly, 
       gr = (int)smem;
     }
     auto &per = G.nb[key];
-    const uint32_t okey = smem * 8u + wpb;
+    const uint32_t okey = smem * 8u + warps;
     auto n_it = per.find(okey);
     if (n_it == per.end()) {
       int v = 0;
-      DG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, kernel, 32 * (int)wpb, smem));
+      DG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, kernel, 32 * (int)warps, smem));
       n_it = per.emplace(okey, v).first;
     }
     nb = n_it->second;
@@ -75,10 +74,10 @@ DgStatus launch_persistent(K kernel, const SearchArgs &a, const WarpLayout &Ly, 
   if (nb <= 0) return fail(DG_ENOTSUP, "search kernel cannot be resident on an SM");
   if (a.occ_pct > 0 && a.occ_pct < 100) nb = std::max(1, (int)((nb * a.occ_pct + 99) / 100));
   int grid = nb * sms;
-  const int need = (int)((a.nq + wpb - 1) / wpb);
+  const int need = (int)((a.nq + queries - 1) / queries);
   if (grid > need) grid = need;
   if (grid < 1) grid = 1;
-  kernel<<<grid, 32 * wpb, smem, st>>>(a, Ly);
+  kernel<<<grid, 32 * warps, smem, st>>>(a, Ly);
   DG_CUDA(cudaGetLastError());
   if (info) {
     info->grid = grid;
@@ -88,49 +87,57 @@ DgStatus launch_persistent(K kernel, const SearchArgs &a, const WarpLayout &Ly, 
   return DG_OK;
 }
 
+template <int NW, int TRAV, int MET, int LPR>
+DgStatus launch_cta(const SearchArgs &a, const WarpLayout &Ly, bool tc, bool filt, cudaStream_t st, LaunchInfo *info) {
+  if constexpr (TRAV == TRAV_BF16) {
+    if (tc) return launch_persistent(beam_search_cta_kernel<NW, TRAV, MET, LPR, true, false>, a, Ly, NW, 1, st, info);
+  }
+  return filt ? launch_persistent(beam_search_cta_kernel<NW, TRAV, MET, LPR, false, true>, a, Ly, NW, 1, st, info)
+              : launch_persistent(beam_search_cta_kernel<NW, TRAV, MET, LPR, false, false>, a, Ly, NW, 1, st, info);
+}
+
+// The CTA-per-query kernel (cta), or the register-list kernel (unfiltered, one
+// seed, beams up to 64).  BF16 rows: beams up to 64 without a filter take the
+// tensor-core distances of the register-list kernel in both (tc), so that a
+// search returns the same bits at every batch size.
 template <int TRAV, int MET, int LPR>
-DgStatus launch_trav(const SearchArgs &a, const WarpLayout &Ly, int lcap, bool filt, cudaStream_t st,
+DgStatus launch_trav(const SearchArgs &a, const WarpLayout &Ly, uint32_t cta, bool tc, bool filt, cudaStream_t st,
                      LaunchInfo *info) {
   constexpr int F = 8;  // lanes per FP32 row in the rerank gather
-  switch (lcap) {
-    case 64:
-      return filt ? launch_persistent(beam_search_kernel<TRAV, MET, LPR, F, 64, true>, a, Ly, st, info)
-                  : launch_persistent(beam_search_kernel<TRAV, MET, LPR, F, 64, false>, a, Ly, st, info);
-    case 256:
-      return filt ? launch_persistent(beam_search_kernel<TRAV, MET, LPR, F, 256, true>, a, Ly, st, info)
-                  : launch_persistent(beam_search_kernel<TRAV, MET, LPR, F, 256, false>, a, Ly, st, info);
-    case 1024:
-      return filt ? launch_persistent(beam_search_kernel<TRAV, MET, LPR, F, 1024, true>, a, Ly, st, info)
-                  : launch_persistent(beam_search_kernel<TRAV, MET, LPR, F, 1024, false>, a, Ly, st, info);
-    default:
-      return fail(DG_EINVAL, "unsupported working-set capacity");
+  if (!cta) {
+    const uint32_t wpb = (a.wpb == 1 || a.wpb == 2) ? a.wpb : 4u;
+    return launch_persistent(beam_search_kernel<TRAV, MET, LPR, F>, a, Ly, wpb, wpb, st, info);
   }
+  return cta == 1   ? launch_cta<1, TRAV, MET, LPR>(a, Ly, tc, filt, st, info)
+         : cta == 2 ? launch_cta<2, TRAV, MET, LPR>(a, Ly, tc, filt, st, info)
+         : cta == 8 ? launch_cta<8, TRAV, MET, LPR>(a, Ly, tc, filt, st, info)
+                    : launch_cta<4, TRAV, MET, LPR>(a, Ly, tc, filt, st, info);
 }
 
 template <int TRAV, int LPR>
-DgStatus launch_met(const SearchArgs &a, const WarpLayout &Ly, int met, int lcap, bool filt,
+DgStatus launch_met(const SearchArgs &a, const WarpLayout &Ly, int met, uint32_t cta, bool tc, bool filt,
                     cudaStream_t st, LaunchInfo *info) {
   switch (met) {
-    case MET_L2: return launch_trav<TRAV, MET_L2, LPR>(a, Ly, lcap, filt, st, info);
-    case MET_DOT: return launch_trav<TRAV, MET_DOT, LPR>(a, Ly, lcap, filt, st, info);
-    default: return launch_trav<TRAV, MET_COS, LPR>(a, Ly, lcap, filt, st, info);
+    case MET_L2: return launch_trav<TRAV, MET_L2, LPR>(a, Ly, cta, tc, filt, st, info);
+    case MET_DOT: return launch_trav<TRAV, MET_DOT, LPR>(a, Ly, cta, tc, filt, st, info);
+    default: return launch_trav<TRAV, MET_COS, LPR>(a, Ly, cta, tc, filt, st, info);
   }
 }
 
 // One entry per traversal kind, defined in its own translation unit.
-DgStatus launch_search_f32(const SearchArgs &a, const WarpLayout &Ly, int met, int lpr, int lcap,
+DgStatus launch_search_f32(const SearchArgs &a, const WarpLayout &Ly, int met, int lpr, uint32_t cta, bool tc,
                            bool filt, cudaStream_t st, LaunchInfo *info);
-DgStatus launch_search_bf16(const SearchArgs &a, const WarpLayout &Ly, int met, int lpr, int lcap,
+DgStatus launch_search_bf16(const SearchArgs &a, const WarpLayout &Ly, int met, int lpr, uint32_t cta, bool tc,
                             bool filt, cudaStream_t st, LaunchInfo *info);
-DgStatus launch_search_f16(const SearchArgs &a, const WarpLayout &Ly, int met, int lpr, int lcap,
+DgStatus launch_search_f16(const SearchArgs &a, const WarpLayout &Ly, int met, int lpr, uint32_t cta, bool tc,
                            bool filt, cudaStream_t st, LaunchInfo *info);
-DgStatus launch_search_int8(const SearchArgs &a, const WarpLayout &Ly, int met, int lpr, int lcap,
+DgStatus launch_search_int8(const SearchArgs &a, const WarpLayout &Ly, int met, int lpr, uint32_t cta, bool tc,
                             bool filt, cudaStream_t st, LaunchInfo *info);
-DgStatus launch_search_pq(const SearchArgs &a, const WarpLayout &Ly, int met, int lpr, int lcap,
+DgStatus launch_search_pq(const SearchArgs &a, const WarpLayout &Ly, int met, int lpr, uint32_t cta, bool tc,
                           bool filt, cudaStream_t st, LaunchInfo *info);
-DgStatus launch_search_rabitq(const SearchArgs &a, const WarpLayout &Ly, int met, int lpr, int lcap,
+DgStatus launch_search_rabitq(const SearchArgs &a, const WarpLayout &Ly, int met, int lpr, uint32_t cta, bool tc,
                               bool filt, cudaStream_t st, LaunchInfo *info);
-DgStatus launch_search_fp8(const SearchArgs &a, const WarpLayout &Ly, int met, int lpr, int lcap,
+DgStatus launch_search_fp8(const SearchArgs &a, const WarpLayout &Ly, int met, int lpr, uint32_t cta, bool tc,
                            bool filt, cudaStream_t st, LaunchInfo *info);
 
 }  // namespace dg

@@ -79,7 +79,8 @@ struct SearchArgs {
   uint32_t *counter;  // work counter, zero at launch
   const uint32_t *perm;  // order in which the grid takes the queries (null = as given)
   uint32_t occ_pct;      // share of the resident CTAs per SM the grid uses (percent; 0 = all)
-  uint32_t wpb;          // warps per CTA of the launch (1, 2 or 4; 0 = 4), one query per warp
+  uint32_t wpb;          // warps per CTA of the register-list kernel (1, 2 or 4; 0 = 4), one query per warp
+  uint32_t limit_smem;   // shared memory that must be available for the search to be accepted
 };
 
 enum TravKind { TRAV_F32 = 0, TRAV_BF16 = 1, TRAV_PQ = 2, TRAV_INT8 = 3, TRAV_RABITQ = 4, TRAV_F16 = 5, TRAV_FP8 = 6 };
@@ -158,9 +159,10 @@ struct Visited {
     const uint32_t h = id * 0x9E3779B1u;
     return B >= 32 ? h : (h & ((1u << B) - 1u));
   }
-  __device__ __forceinline__ void clear(int lane) const {
+  // by `step` threads, numbered t
+  __device__ __forceinline__ void clear(int t, int step = 32) const {
     const uint32_t words = 1u << bbits, empty = tagged() ? 0u : 0xFFFFFFFFu;
-    for (uint32_t i = lane; i < words; i += 32) w[i] = empty;
+    for (uint32_t i = t; i < words; i += step) w[i] = empty;
   }
   // True when `id` is recorded; otherwise records it.
   __device__ __forceinline__ bool test_and_set(uint32_t id) const {
@@ -803,9 +805,10 @@ __device__ __forceinline__ float int8_decode_group(const uint8_t *__restrict__ c
 // ------------------------------------------------------------ quantizers
 // PQ lookup table (src/pq.rs:181-198): lut[m][c] = sequential f32 sum of
 // squared differences over the subspace, rounded like the oracle.
-__device__ __forceinline__ void build_pq_lut(const SearchArgs &a, const float *qs, float *lut, int lane) {
+// (By `step` threads, numbered t.)
+__device__ __forceinline__ void build_pq_lut(const SearchArgs &a, const float *qs, float *lut, int t0, int step = 32) {
   const uint32_t total = a.pq_M * a.pq_K;
-  for (uint32_t e = lane; e < total; e += 32) {
+  for (uint32_t e = t0; e < total; e += step) {
     const uint32_t m = e / a.pq_K;
     const float *cen = a.pq_cb + (size_t)e * a.pq_ds;
     const float *qq = qs + m * a.pq_ds;
@@ -821,18 +824,19 @@ __device__ __forceinline__ void build_pq_lut(const SearchArgs &a, const float *q
 __device__ __forceinline__ float pq_adc(const SearchArgs &a, const float *lut, uint32_t id) {
   const uint8_t *row = a.codes + (size_t)id * a.code_stride;
   float d = 0.0f;
-  const uint32_t K = a.pq_K;
-  uint32_t m = 0;
-  for (uint32_t c = 0; m < a.pq_M; ++c) {
-    const uint4 v = __ldg(reinterpret_cast<const uint4 *>(row) + c);
+  const uint32_t K = a.pq_K, M = a.pq_M;
+  for (uint32_t m0 = 0; m0 < M; m0 += 16) {
+    const uint4 v = __ldg(reinterpret_cast<const uint4 *>(row) + m0 / 16);
     const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+    const float *t = lut + m0 * K;
+    if (m0 + 16 <= M) {  // sixteen independent look-ups, then the sum in order
+      float x[16];
 #pragma unroll
-    for (int b = 0; b < 16; ++b) {
-      if (m < a.pq_M) {
-        const uint32_t code = (w[b >> 2] >> (8 * (b & 3))) & 0xffu;
-        d = __fadd_rn(d, lut[m * K + code]);
-        ++m;
-      }
+      for (int b = 0; b < 16; ++b, t += K) x[b] = t[(w[b >> 2] >> (8 * (b & 3))) & 0xffu];
+#pragma unroll
+      for (int b = 0; b < 16; ++b) d = __fadd_rn(d, x[b]);
+    } else {
+      for (uint32_t b = 0; b < M - m0; ++b, t += K) d = __fadd_rn(d, t[(w[b >> 2] >> (8 * (b & 3))) & 0xffu]);
     }
   }
   return d;
@@ -842,9 +846,10 @@ __device__ __forceinline__ float pq_adc(const SearchArgs &a, const float *lut, u
 // the code (centroid concatenation, src/pq.rs:151-160) and evaluates the metric
 // (src/quantized.rs:28-36); q . decode(code) = sum_m ip[m][code_m] with
 // ip[m][c] = q_m . centroid(m, c).
-__device__ __forceinline__ void build_pq_ip_lut(const SearchArgs &a, const float *qs, float *lut, int lane) {
+__device__ __forceinline__ void build_pq_ip_lut(const SearchArgs &a, const float *qs, float *lut, int t0,
+                                                int step = 32) {
   const uint32_t total = a.pq_M * a.pq_K;
-  for (uint32_t e = lane; e < total; e += 32) {
+  for (uint32_t e = t0; e < total; e += step) {
     const uint32_t m = e / a.pq_K;
     const float *cen = a.pq_cb + (size_t)e * a.pq_ds;
     const float *qq = qs + m * a.pq_ds;

@@ -1,6 +1,6 @@
 // dg_search_kernel.cuh -- the persistent beam-search kernel template.
 #pragma once
-#include "dg_search.cuh"
+#include "dg_search_tile16.cuh"
 
 namespace dg {
 
@@ -26,10 +26,10 @@ struct QueryCtx {
 };
 
 // Distances for the cnt staged candidates (lane j holds cand), per traversal
-// kind.  TC selects tensor-core BF16 distances (the register-list kernel);
-// the general kernel, with more state per warp, computes them as packed FP32
-// FMAs, which measured faster there.
-template <int TRAV, int MET, int LPR, bool TC = true>
+// kind.  TC selects tensor-core BF16 distances (beams up to 64, no filter);
+// searches with filters or beams above 64 compute them as packed FP32 FMAs.
+// H16: at most 16 candidates, more loads in flight (dg_search_tile16.cuh).
+template <int TRAV, int MET, int LPR, bool TC = true, bool H16 = false>
 __device__ __forceinline__ float batch_distance(const SearchArgs &a, uint8_t *wsm,
                                                 const WarpLayout &Ly, uint32_t cand, int cnt,
                                                 int lane, float qq) {
@@ -43,7 +43,8 @@ __device__ __forceinline__ float batch_distance(const SearchArgs &a, uint8_t *ws
     const uint8_t *qhl = wsm + Ly.prov;
     const float2 qs2 = *reinterpret_cast<const float2 *>(wsm + Ly.prov + 2 * a.dpad);  // (s_q, |q|^2)
     const float2 sn = lane < cnt ? __ldg(a.fp8_sn + cand) : make_float2(0.0f, 0.0f);
-    const float dot = sn.x * qs2.x * fp8_dot_mma(a.vec_fp8, a.dpad, qhl, cand, cnt, lane);
+    const float dot = sn.x * qs2.x * (H16 ? fp8_dot_mma16(a, qhl, cand, cnt, lane)
+                                          : fp8_dot_mma(a.vec_fp8, a.dpad, qhl, cand, cnt, lane));
     if (MET == MET_L2) return finish_metric(MET, sqrt_l2, fmaxf(qs2.y + sn.y - 2.0f * dot, 0.0f), 0.0f, qq);
     return finish_metric(MET, false, dot, sn.y, qq);
   } else if (TRAV == TRAV_BF16 && !TC) {
@@ -54,7 +55,8 @@ __device__ __forceinline__ float batch_distance(const SearchArgs &a, uint8_t *ws
     const uint16_t *qhl = reinterpret_cast<const uint16_t *>(wsm + Ly.prov);
     const float q2 = *reinterpret_cast<const float *>(wsm + Ly.prov + 4 * a.dpad);
     const float xx = lane < cnt ? __ldg(a.bf16_n2 + cand) : 0.0f;
-    const float dot = bf16_dot_mma(a.vec_bf16, a.dpad, qhl, cand, cnt, lane);
+    const float dot = H16 ? bf16_dot_mma16(a, qhl, cand, cnt, lane)
+                          : bf16_dot_mma(a.vec_bf16, a.dpad, qhl, cand, cnt, lane);
     if (MET == MET_L2) return finish_metric(MET, sqrt_l2, fmaxf(__fsub_rn(__fadd_rn(q2, xx), 2.0f * dot), 0.0f),
                                             0.0f, qq);
     return finish_metric(MET, false, dot, xx, qq);
@@ -68,7 +70,8 @@ __device__ __forceinline__ float batch_distance(const SearchArgs &a, uint8_t *ws
     if (MET == MET_L2) {
       const uint8_t *qc = wsm + Ly.prov;
       const uint32_t qn = *reinterpret_cast<const uint32_t *>(qc + align16(a.dpad));
-      const uint32_t s = int8_l2_mma(a.codes, a.code_stride, qc, qn, a.i8_norm, cand, cnt, lane);
+      const uint32_t s = H16 ? int8_l2_mma16(a, qc, qn, cand, cnt, lane)
+                             : int8_l2_mma(a.codes, a.code_stride, qc, qn, a.i8_norm, cand, cnt, lane);
       float d = __fmul_rn(__fmul_rn(__uint2float_rn(s), a.i8_scale), a.i8_scale);
       return sqrt_l2 ? __fsqrt_rn(d) : d;
     } else {
@@ -79,7 +82,8 @@ __device__ __forceinline__ float batch_distance(const SearchArgs &a, uint8_t *ws
       const double2 qp = *reinterpret_cast<const double2 *>(qd + 4 * ds);  // (q scale, sum q)
       const uint32_t c2 = lane < cnt ? __ldg(a.i8_norm + cand) : 0u;
       const uint32_t c1 = lane < cnt ? __ldg(a.i8_sum + cand) : 0u;
-      const double qc = int8_dot_mma(a.codes, a.code_stride, qd, ds, cand, cnt, lane) * qp.x;
+      const double qc = (H16 ? int8_dot_mma16(a, qd, ds, cand, cnt, lane)
+                             : int8_dot_mma(a.codes, a.code_stride, qd, ds, cand, cnt, lane)) * qp.x;
       const double sc = a.i8_scale, of = a.i8_offset;
       const float dot = (float)(sc * qc + of * qp.y);
       const float vv = MET == MET_COS ? (float)(sc * sc * (double)c2 + 2.0 * sc * of * (double)c1 +
@@ -393,7 +397,8 @@ __device__ __forceinline__ void reg_insert(const uint64_t *skeys, int ns, uint64
 // Unfiltered search with beams up to 64: the working list lives in registers,
 // entry i in lane i % 32 (w0 for i < 32, w1 above), so finding the frontier,
 // the threshold and insertion ranks are ballots and shuffles instead of
-// shared-memory binary searches.  Results are identical to search_one.
+// shared-memory binary searches.  Results are identical to search_cta
+// (dg_search_cta.cuh), which takes the other searches and small batches.
 template <int TRAV, int MET, int LPR, int LPRF>
 __device__ inline void search_one_reg(const SearchArgs &a, uint32_t q, uint8_t *wsm, const WarpLayout &Ly,
                                       int lane) {
@@ -480,143 +485,12 @@ __device__ inline void search_one_reg(const SearchArgs &a, uint32_t q, uint8_t *
                                 qs, qq, n_exp, n_dist, lane);
 }
 
-template <int TRAV, int MET, int LPR, int LPRF, int LCAP, bool FILT>
-__device__ inline void search_one(const SearchArgs &a, uint32_t q, uint8_t *wsm, const WarpLayout &Ly,
-                           int lane) {
-  uint64_t *W[2] = {reinterpret_cast<uint64_t *>(wsm + Ly.w0), reinterpret_cast<uint64_t *>(wsm + Ly.w1)};
-  uint64_t *RES = reinterpret_cast<uint64_t *>(wsm + Ly.res);
-  uint64_t *cst = reinterpret_cast<uint64_t *>(wsm + Ly.cstage);
-  uint32_t *stage = reinterpret_cast<uint32_t *>(wsm + Ly.stage);
-  const Visited vt{reinterpret_cast<uint32_t *>(wsm + Ly.hash), a.hbits, a.hB};
-  float *qs = reinterpret_cast<float *>(wsm + Ly.qf);
-
-  const uint32_t L = a.perL ? a.perL[q] : a.L;
-  const uint32_t k = a.perK ? a.perK[q] : a.k;
-  // every traversal other than exact FP32 can be reranked with FP32 rows
-  const bool use_rerank = TRAV != TRAV_F32 && a.rerank > 0;
-  const uint32_t search_k = use_rerank ? max(a.rerank, k) : k;
-
-  // per-query filter program
-  QueryCtx qc{a.fops, a.fnops};
-  if (a.foffs) {
-    qc.fops = a.fops + a.foffs[q];
-    qc.fnops = a.foffs[q + 1] - a.foffs[q];
-  }
-  const bool labeled = FILT && qc.fnops > 0;
-  const bool tombed = FILT && a.tomb != nullptr;
-  const bool filtered = labeled || tombed;
-  uint32_t working = L, max_iter = 0xffffffffu;
-  if (labeled) {  // src/filtered.rs:35-56, src/incremental.rs:1048-1062
-    working = max(L * 4, k * 10);
-    max_iter = working * 2;
-  } else if (tombed) {  // tombstone_config (src/incremental.rs:505-516)
-    working = max(L * 2, search_k + min(a.ntomb, L));
-    max_iter = working * 2;
-  }
-  const bool two = a.seed2 != DG_PAD && a.seed2 != a.medoid;
-  if (two) working = max(working, 2u);  // both seeds enter w (src/lib.rs:218-229)
-
-  // ---- query into shared memory (zero padded), norms, visited table
-  const float *qg = a.Q + (size_t)q * a.d;
-  for (uint32_t i = lane; i < a.dpad; i += 32) qs[i] = i < a.d ? qg[i] : 0.0f;
-  vt.clear(lane);
-  __syncwarp();
-  float qq = 0.0f;
-  if (MET == MET_COS) qq = query_norm2<TRAV>(qs, a.d, lane);
-  prepare_query<TRAV, MET>(a, wsm, Ly, qs, lane);
-
-  const uint64_t *labels = a.labels;
-  // a result must be live (UnifiedView::is_live, src/incremental.rs:463-470) and match
-  auto allow = [&](uint32_t id) -> bool {
-    if (a.tomb && ((__ldg(a.tomb + (id >> 5)) >> (id & 31)) & 1u)) return false;
-    return !labeled || filter_eval(qc.fops, qc.fnops, a.fpool, labels + (size_t)id * a.nf, a.nf);
-  };
-
-  // ---- seed: the medoid (DiskANN::search_with_dists seeds [medoid])
-  int cur = 0, wsize = 0, rsize = 0;
-  uint32_t n_exp = 0, n_dist = 0;
-  // merges this lane's match key (kKeyInvalid = none) into the result list
-  auto add_results = [&](uint64_t mk) {
-    const int nm = prepare_batch(mk, RES, rsize, (int)search_k, cst, lane);
-    if (nm > 0) {
-      // merge in place through the non-current w buffer as scratch
-      uint64_t *tmp = W[cur ^ 1];
-      rsize = merge_keys(RES, rsize, tmp, (int)search_k, cst, nm, lane);
-      for (int i = lane; i < rsize; i += 32) RES[i] = tmp[i];
-      __syncwarp();
-    }
-  };
-  // ---- seeds: the medoid, and the delta layer's entry point of a base +
-  // delta index (UnifiedView::entry_points, src/incremental.rs:383-392).  They
-  // are the first staged batch the loop merges (src/lib.rs:218-233).
-  int ns = two ? 2 : 1;
-  if (lane == 0) {
-    stage[0] = a.medoid;
-    vt.test_and_set(a.medoid);
-    if (two) {
-      stage[1] = a.seed2;
-      vt.test_and_set(a.seed2);
-    }
-  }
-  __syncwarp();
-
-  while (true) {
-    n_dist += ns;
-    // ---- distances and merge, 32 candidates at a time
-    for (int g0 = 0; g0 < ns; g0 += 32) {
-      const int cnt = min(32, ns - g0);
-      const uint32_t cand = lane < cnt ? stage[g0 + lane] : DG_PAD;
-      float d = batch_distance<TRAV, MET, LPR, false>(a, wsm, Ly, cand, cnt, lane, qq);
-      if (TRAV != TRAV_F32 && a.code_limit < a.n && lane < cnt && cand >= a.code_limit)
-        d = exact_row_distance<MET>(a, qs, cand, qq);
-      uint64_t key = lane < cnt ? make_key(d, cand) : kKeyInvalid;
-      bool match = false;
-      if (filtered && lane < cnt) match = allow(cand);
-      insert_batch(key, W, cur, wsize, (int)working, cst, lane);
-      // result list: every visited match, kept as the search_k smallest
-      if (filtered) add_results((lane < cnt && match) ? make_key(d, cand) : kKeyInvalid);
-    }
-
-    // first unexpanded entry of w (the frontier minimum)
-    int idx = -1;
-    for (int base = 0; base < wsize; base += 32) {
-      const int i = base + lane;
-      const bool un = i < wsize && !key_expanded(W[cur][i]);
-      const uint32_t m = __ballot_sync(kFull, un);
-      if (m) {
-        idx = base + __ffs(m) - 1;
-        break;
-      }
-    }
-    if (idx < 0) break;
-    const uint64_t best = W[cur][idx];
-    const float bd = key_dist(best);
-    if (filtered) {
-      if (n_exp >= max_iter) break;  // src/lib.rs:237-240
-      if (rsize >= (int)search_k && search_k > 0) {  // :242-251
-        const float worst = key_dist(RES[search_k - 1]);
-        if (worst >= 0.0f && bd > __fmul_rn(worst, 1.5f)) break;
-      }
-    }
-    if (wsize >= (int)working && bd >= key_dist(W[cur][working - 1])) break;  // :253-259
-    if (lane == 0) W[cur][idx] = best | 1ull;
-    ++n_exp;
-
-    // ---- stage unvisited neighbours
-    ns = stage_neighbours(a, a.adj + (size_t)key_id(best) * a.R, vt, stage, lane);
-  }
-
-  // ---- emit
-  emit_results<TRAV, MET, LPRF>(a, q, filtered ? RES : W[cur], filtered ? rsize : wsize, use_rerank, search_k,
-                                W[cur ^ 1], qs, qq, n_exp, n_dist, lane);
-}
-
 // Resident blocks per SM the register allocation is sized for (4 warps each).
 #ifndef DG_SEARCH_MIN_BLOCKS
 #define DG_SEARCH_MIN_BLOCKS 6
 #endif
 
-template <int TRAV, int MET, int LPR, int LPRF, int LCAP, bool FILT>
+template <int TRAV, int MET, int LPR, int LPRF>
 __global__ void __launch_bounds__(128, DG_SEARCH_MIN_BLOCKS) beam_search_kernel(SearchArgs a, WarpLayout Ly) {
   extern __shared__ __align__(16) uint8_t smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -627,10 +501,7 @@ __global__ void __launch_bounds__(128, DG_SEARCH_MIN_BLOCKS) beam_search_kernel(
     q = __shfl_sync(kFull, q, 0);
     if (q >= a.nq) break;
     if (a.perm) q = __ldg(a.perm + q);
-    if (LCAP == 64 && !FILT)
-      search_one_reg<TRAV, MET, LPR, LPRF>(a, q, wsm, Ly, lane);
-    else
-      search_one<TRAV, MET, LPR, LPRF, LCAP, FILT>(a, q, wsm, Ly, lane);
+    search_one_reg<TRAV, MET, LPR, LPRF>(a, q, wsm, Ly, lane);
   }
 }
 

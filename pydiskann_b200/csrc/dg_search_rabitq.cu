@@ -4,9 +4,9 @@
 // src/quantized.rs:28-36).
 #include "dg_launch.cuh"
 namespace dg {
-DgStatus launch_search_rabitq(const SearchArgs &a, const WarpLayout &Ly, int met, int lpr, int lcap,
+DgStatus launch_search_rabitq(const SearchArgs &a, const WarpLayout &Ly, int met, int lpr, uint32_t cta, bool tc,
                               bool filt, cudaStream_t st, LaunchInfo *info) {
   (void)lpr;
-  return launch_met<TRAV_RABITQ, 1>(a, Ly, met, lcap, filt, st, info);
+  return launch_met<TRAV_RABITQ, 1>(a, Ly, met, cta, tc, filt, st, info);
 }
 }  // namespace dg

@@ -464,6 +464,222 @@ __global__ void __launch_bounds__(256) k_exact_knn(const float *X, uint64_t n, u
   }
 }
 
+// Tiled form for k <= kKnnTileK: a CTA takes 64 queries and a slice of the
+// rows, 64 at a time; each thread owns a 4 x 4 tile of (query, row) pairs in
+// FP64 registers, fed from shared memory that holds 16 coordinates of both
+// sides as doubles (converted once per CTA instead of once per pair).  Every
+// pair is summed in coordinate order with one rounding per operation, as the
+// kernel above does, so the results are the same bits.  The distances of a
+// tile go through shared memory to the warps, each keeping the k best keys of
+// eight queries; entries beyond the smallest k-th distance any slice has seen
+// (qthr) are dropped before insertion, and k_knn_merge joins the slices' lists.
+// Bound by the FP64 pipe: a subtraction and an FMA per coordinate and pair,
+// 1.4 ms for 1000 queries x 100k x 128 at 64 lanes per SM; the kernel above ran
+// 125 CTAs of 8 warps and converted both operands of every pair.
+constexpr int kKnnT = 64, kKnnJ = 16, kKnnTileK = 128;
+constexpr int kKnnS = kKnnT + 2;  // row of 64 doubles, padded
+
+template <bool L2>
+__global__ void __launch_bounds__(256, 2) k_knn_tiled(const float *__restrict__ X, uint64_t n, uint32_t d,
+                                                      uint32_t dpad, const float *__restrict__ Q, uint32_t nq,
+                                                      uint32_t k, int metric, uint32_t kcap, uint64_t rows_per_slice,
+                                                      uint32_t *qthr, uint64_t *part, uint32_t *part_cnt) {
+  extern __shared__ __align__(16) uint8_t sm[];
+  double *xs = reinterpret_cast<double *>(sm);                        // [kKnnJ][kKnnS]
+  double *qs = xs + kKnnJ * kKnnS;                                    // [kKnnJ][kKnnS]
+  float *dist = reinterpret_cast<float *>(qs + kKnnJ * kKnnS);        // [kKnnT queries][kKnnT + 1 rows]
+  uint64_t *cst = reinterpret_cast<uint64_t *>(sm + align16(2 * kKnnJ * kKnnS * 8 + kKnnT * (kKnnT + 1) * 4));  // [8][32]
+  uint64_t *lists = cst + 8 * 32;                                     // [kKnnT][2][kcap]
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tx = tid & 15, ty = tid >> 4;  // rows tx + 16 i, queries ty + 16 i
+  const uint32_t q0 = blockIdx.x * kKnnT;
+  const uint64_t x0 = blockIdx.y * rows_per_slice, x1 = min(n, x0 + rows_per_slice);
+  // loads: thread t takes coordinates 4 (t % 4) .. +3 of row / query t / 4
+  const int lr = tid >> 2, lc = (tid & 3) * 4;
+  int cur[8] = {}, size[8] = {};  // this warp's queries 8 warp + u
+  for (uint64_t base = x0; base < x1; base += kKnnT) {
+    double s[4][4], nx[4], nq_[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      nx[i] = nq_[i] = 0.0;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) s[i][j] = 0.0;
+    }
+    float4 xv, qv;
+    auto fetch = [&](uint32_t j0) {
+      xv = qv = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      if (base + lr < x1 && j0 + lc < dpad) xv = __ldg(reinterpret_cast<const float4 *>(X + (base + lr) * dpad + j0 + lc));
+      if (q0 + lr < nq) {
+        const float *q = Q + (size_t)(q0 + lr) * d + j0 + lc;
+        if (j0 + lc < d) qv.x = __ldg(q);
+        if (j0 + lc + 1 < d) qv.y = __ldg(q + 1);
+        if (j0 + lc + 2 < d) qv.z = __ldg(q + 2);
+        if (j0 + lc + 3 < d) qv.w = __ldg(q + 3);
+      }
+    };
+    fetch(0);
+    for (uint32_t j0 = 0; j0 < d; j0 += kKnnJ) {
+      __syncthreads();  // the previous chunk (and the previous tile's distances) are consumed
+      const float xa[4] = {xv.x, xv.y, xv.z, xv.w}, qa[4] = {qv.x, qv.y, qv.z, qv.w};
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        xs[(lc + e) * kKnnS + lr] = (double)xa[e];
+        qs[(lc + e) * kKnnS + lr] = (double)qa[e];
+      }
+      __syncthreads();
+      if (j0 + kKnnJ < d) fetch(j0 + kKnnJ);  // in flight under the arithmetic
+#pragma unroll 4
+      for (int j = 0; j < kKnnJ; ++j) {
+        double xr[4], qr[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          xr[i] = xs[j * kKnnS + tx + 16 * i];
+          qr[i] = qs[j * kKnnS + ty + 16 * i];
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            if (L2) {
+              const double t = qr[i] - xr[c];
+              s[i][c] = fma(t, t, s[i][c]);
+            } else {
+              s[i][c] = fma(qr[i], xr[c], s[i][c]);
+            }
+          }
+          if (!L2) {
+            nx[i] = fma(xr[i], xr[i], nx[i]);
+            nq_[i] = fma(qr[i], qr[i], nq_[i]);
+          }
+        }
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        double v = s[i][c];
+        if (L2) {
+          if (metric == DG_L2) v = sqrt(v);
+        } else if (metric == DG_COSINE) {
+          v = (nq_[i] == 0.0 || nx[c] == 0.0) ? 1.0 : 1.0 - v / (sqrt(nq_[i]) * sqrt(nx[c]));
+        } else {
+          v = 1.0 - v;
+        }
+        dist[(ty + 16 * i) * (kKnnT + 1) + tx + 16 * c] = (float)v;
+      }
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      const uint32_t ql = 8 * warp + u, q = q0 + ql;
+      if (q >= nq) break;
+      uint64_t *const bufs[2] = {lists + (size_t)ql * 2 * kcap, lists + (size_t)ql * 2 * kcap + kcap};
+      const uint32_t tb = *reinterpret_cast<volatile uint32_t *>(qthr + q);
+      const uint64_t worst = size[u] >= (int)k ? bufs[cur[u]][k - 1] : kKeyInvalid;
+      uint64_t key[2];
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const uint64_t r = base + lane + 32 * h;
+        key[h] = r < x1 ? make_key(dist[ql * (kKnnT + 1) + lane + 32 * h], (uint32_t)r) : kKeyInvalid;
+        if (key_hi(key[h]) > tb || key[h] >= worst) key[h] = kKeyInvalid;
+      }
+      if (!__any_sync(kFull, key[0] != kKeyInvalid || key[1] != kKeyInvalid)) continue;
+      insert_batch(key[0], bufs, cur[u], size[u], (int)k, cst + 32 * warp, lane);
+      insert_batch(key[1], bufs, cur[u], size[u], (int)k, cst + 32 * warp, lane);
+      if (size[u] >= (int)k && lane == 0) {
+        const uint32_t nb = key_hi(bufs[cur[u]][k - 1]);
+        if (nb < tb) atomicMin(qthr + q, nb);
+      }
+    }
+  }
+#pragma unroll
+  for (int u = 0; u < 8; ++u) {
+    const uint32_t ql = 8 * warp + u, q = q0 + ql;
+    if (q >= nq) break;
+    const uint64_t *l = lists + (size_t)ql * 2 * kcap + (size_t)cur[u] * kcap;
+    const size_t at = (size_t)blockIdx.y * nq + q;
+    for (int i = lane; i < size[u]; i += 32) part[at * k + i] = l[i];
+    if (lane == 0) part_cnt[at] = (uint32_t)size[u];
+  }
+}
+
+// The k smallest keys of a query's slice lists (a warp per query).
+__global__ void __launch_bounds__(128) k_knn_merge(const uint64_t *part, const uint32_t *part_cnt, uint32_t slices,
+                                                   uint32_t nq, uint32_t k, uint32_t *out_ids, float *out_d) {
+  __shared__ uint64_t buf[4][2][kKnnTileK];
+  __shared__ uint64_t cst[4][32];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  uint64_t *const bufs[2] = {buf[warp][0], buf[warp][1]};
+  for (uint32_t q = blockIdx.x * 4 + warp; q < nq; q += gridDim.x * 4) {
+    int cur = 0, size = 0;
+    for (uint32_t sl = 0; sl < slices; ++sl) {
+      const size_t at = (size_t)sl * nq + q;
+      const uint32_t c = part_cnt[at];
+      for (uint32_t j0 = 0; j0 < c; j0 += 32) {
+        const uint32_t j = j0 + lane;
+        insert_batch(j < c ? part[at * k + j] : kKeyInvalid, bufs, cur, size, (int)k, cst[warp], lane);
+      }
+    }
+    for (int i = lane; i < (int)k; i += 32) {
+      out_ids[(size_t)q * k + i] = i < size ? key_id(bufs[cur][i]) : DG_PAD;
+      out_d[(size_t)q * k + i] = i < size ? key_dist(bufs[cur][i]) : __int_as_float(0x7f800000);
+    }
+    __syncwarp();
+  }
+}
+
+// Launches the tiled kNN: the rows are cut into the number of slices that
+// leaves the fewest tiles to the busiest of the 2 CTAs per SM.
+static DgStatus knn_tiled(const float *v, uint64_t n, uint32_t dim, uint32_t dpad, const float *q, uint32_t nq,
+                          uint32_t k, int metric, uint32_t *oi, float *od, cudaStream_t st) {
+  int dev = 0, sms = 0;
+  DG_CUDA(cudaGetDevice(&dev));
+  DG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  uint32_t kcap = 16;
+  while (kcap < k) kcap <<= 1;
+  const size_t smem = align16(2 * kKnnJ * kKnnS * 8 + kKnnT * (kKnnT + 1) * 4) + 8 * 32 * 8 + (size_t)kKnnT * 2 * kcap * 8;
+  const uint64_t qb = (nq + kKnnT - 1) / kKnnT, tiles = (n + kKnnT - 1) / kKnnT, slots = 2ull * sms;
+  uint64_t best = ~0ull, slices = 1;
+  for (uint64_t s = 1; s <= std::min<uint64_t>(tiles, 4 * slots); ++s) {
+    const uint64_t cost = ((qb * s + slots - 1) / slots) * ((tiles + s - 1) / s + 2);
+    if (cost < best) {
+      best = cost;
+      slices = s;
+    }
+  }
+  const uint64_t rows = (tiles + slices - 1) / slices * kKnnT;
+  slices = (n + rows - 1) / rows;
+  uint32_t *thr = nullptr, *pc = nullptr;
+  uint64_t *part = nullptr;
+  if (cudaMallocAsync(&thr, (size_t)nq * 4, st) != cudaSuccess ||
+      cudaMallocAsync(&pc, (size_t)slices * nq * 4, st) != cudaSuccess ||
+      cudaMallocAsync(&part, (size_t)slices * nq * k * 8, st) != cudaSuccess) {
+    for (void *p : {(void *)thr, (void *)pc, (void *)part})
+      if (p) cudaFreeAsync(p, st);
+    return fail(DG_ENOMEM, "exact knn staging");
+  }
+  const bool l2 = metric == DG_L2SQ || metric == DG_L2;
+  auto kern = l2 ? k_knn_tiled<true> : k_knn_tiled<false>;
+  DgStatus s = DG_OK;
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e == cudaSuccess) e = cudaMemsetAsync(thr, 0xff, (size_t)nq * 4, st);
+  if (e == cudaSuccess) {
+    kern<<<dim3((unsigned)qb, (unsigned)slices), 256, smem, st>>>(v, n, dim, dpad, q, nq, k, metric, kcap, rows, thr,
+                                                                  part, pc);
+    e = cudaGetLastError();
+  }
+  if (e == cudaSuccess) {
+    k_knn_merge<<<(unsigned)std::min<uint32_t>((nq + 3) / 4, 148 * 16), 128, 0, st>>>(part, pc, (uint32_t)slices, nq, k,
+                                                                                   oi, od);
+    e = cudaGetLastError();
+  }
+  if (e != cudaSuccess) s = cuda_fail(e, "exact knn launch");
+  cudaFreeAsync(thr, st);
+  cudaFreeAsync(pc, st);
+  cudaFreeAsync(part, st);
+  return s;
+}
+
 // ------------------------------------------------------------ PQ training
 // ProductQuantizer::train (src/pq.rs:51-119): per subspace, k-means++ seeding
 // then Lloyd iterations; empty clusters restart from a random training point.
@@ -793,7 +1009,9 @@ DgStatus dg_exact_knn(const float *X, uint64_t n, uint32_t dim, const float *Q, 
     s = fail(DG_ENOMEM, "exact knn staging");
   if (s == DG_OK) s = upload_rows_f32(X, n, dim, dpad, v, st);
   if (s == DG_OK) cudaMemcpyAsync(q, Q, (size_t)nq * dim * 4, cudaMemcpyHostToDevice, st);
-  if (s == DG_OK) {
+  if (s == DG_OK && k <= (uint32_t)kKnnTileK) {
+    s = knn_tiled(v, n, dim, dpad, q, nq, k, metric, oi, od, st);
+  } else if (s == DG_OK) {  // longer lists than a 64-query CTA can hold: 8 queries per CTA
     uint32_t kcap = 32;
     while (kcap < k) kcap <<= 1;
     const size_t smem = align16((32 * (dim + 1) + kKnnWarps * dim) * 4) + (size_t)kKnnWarps * (2 * kcap + 32) * 8;

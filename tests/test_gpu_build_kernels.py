@@ -1,0 +1,35 @@
+"""Exact kNN and PQ kernels at the edges of their tiles, against the CPU oracle.
+
+Integer-valued data: distances, running sums and cluster sums are exact in any
+order, so ids, codes and codebooks must equal the oracle's bit for bit.
+"""
+import numpy as np
+import pytest
+
+import pydiskann_b200 as dg
+from pydiskann_b200 import synth
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n,d,nq,k", [(1, 1, 1, 1), (63, 33, 64, 5), (65, 16, 65, 16), (700, 100, 3, 128),
+                                      (700, 20, 70, 129), (5000, 48, 200, 17)])
+@pytest.mark.parametrize("metric", ["l2", "euclidean"])
+def test_exact_knn_edges(oracle, n, d, nq, k, metric):
+    X = synth.mixture(n, d, 4, seed=3)
+    Q = synth.mixture(nq, d, 4, seed=3, stream=synth.STREAM_QUERY)
+    gi, gd = dg.exact_knn(X, Q, k, metric)
+    oi, od = oracle.exact_knn(X, Q, k)
+    if metric == "euclidean":
+        od = np.sqrt(od.astype(np.float64)).astype(np.float32)
+    assert np.array_equal(gi, oi) and np.array_equal(gd, od)
+
+
+def test_exact_knn_cosine_against_float64():
+    X = np.random.default_rng(0).standard_normal((3000, 72)).astype(np.float32)
+    Q = np.random.default_rng(1).standard_normal((90, 72)).astype(np.float32)
+    _, gd = dg.exact_knn(X, Q, 10, "cosine")
+    Xd, Qd = X.astype(np.float64), Q.astype(np.float64)
+    D = 1.0 - Qd @ Xd.T / (np.linalg.norm(Qd, axis=1)[:, None] * np.linalg.norm(Xd, axis=1)[None])
+    # the FP64 value rounded to FP32, and the FP64 sums' own rounding of up to 72 terms
+    assert np.abs(gd - np.sort(D, axis=1)[:, :10]).max() <= 2.0 ** -24 + 72 * 2.0 ** -50

@@ -70,9 +70,11 @@ __global__ void k_int8_norm(const uint8_t *codes, uint64_t n, uint32_t stride, u
     if (sums) sums[r] = t;
   }
 }
-// ProductQuantizer::encode (src/pq.rs:122-149): argmin with strict '<'.
+// ProductQuantizer::encode (src/pq.rs:122-149): argmin with strict '<', each
+// distance summed in coordinate order.  Row i's code of subspace m goes to
+// codes[i * row_step + m * sub_step].  Any subspace width.
 __global__ void k_pq_encode(const float *v, uint64_t n, uint32_t dpad, uint32_t M, uint32_t K,
-                            uint32_t ds, const float *cb, uint8_t *codes, uint32_t stride) {
+                            uint32_t ds, const float *cb, uint8_t *codes, uint64_t row_step, uint64_t sub_step) {
   const uint32_t m = blockIdx.y;
   for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n;
        i += (uint64_t)gridDim.x * blockDim.x) {
@@ -91,8 +93,92 @@ __global__ void k_pq_encode(const float *v, uint64_t n, uint32_t dpad, uint32_t 
         bc = c;
       }
     }
-    codes[i * stride + m] = (uint8_t)bc;
+    codes[i * row_step + m * sub_step] = (uint8_t)bc;
   }
+}
+
+// The same for the usual widths: the subspace's codebook sits in shared
+// memory, two centroids interleaved, a thread holds two sub-vectors in
+// registers, and each packed instruction serves two centroids (a subtraction,
+// a multiplication and an addition per coordinate, each rounded once, in
+// coordinate order: the same bits).  Bound by FP32 issue; the kernel above
+// re-reads the sub-vector and the centroid for every term (200k rows, M = 16,
+// K = 256, 8 wide: 24 ms).
+template <int DS>
+__global__ void __launch_bounds__(256) k_pq_nearest(const float *__restrict__ v, uint64_t n, uint32_t stride,
+                                                    uint32_t K, const float *__restrict__ cb, uint8_t *codes,
+                                                    uint64_t row_step, uint64_t sub_step) {
+  __shared__ __align__(16) float2 cs[128 * DS];  // [pair of centroids][coordinate]
+  const uint32_t m = blockIdx.y, pairs = (K + 1) / 2;
+  const float inf = __int_as_float(0x7f800000);
+  for (uint32_t e = threadIdx.x; e < pairs * DS; e += blockDim.x) {
+    const uint32_t c = 2 * (e / DS), j = e % DS;
+    const float *p = cb + ((size_t)m * K + c) * DS + j;
+    cs[e] = make_float2(p[0], c + 1 < K ? p[DS] : inf);  // (an infinite distance is never the smallest)
+  }
+  __syncthreads();
+  const float2 neg1 = make_float2(-1.0f, -1.0f);
+  const uint64_t step = (uint64_t)gridDim.x * blockDim.x;
+  for (uint64_t i0 = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i0 < n; i0 += 2 * step) {
+    const uint64_t i1 = i0 + step < n ? i0 + step : i0;
+    const float *x0 = v + i0 * stride + m * DS, *x1 = v + i1 * stride + m * DS;
+    float a[DS], b[DS];
+    if (DS % 4 == 0) {  // stride and the subspace's offset are then multiples of 16 bytes
+#pragma unroll
+      for (int j = 0; j < DS / 4; ++j) {
+        reinterpret_cast<float4 *>(a)[j] = __ldg(reinterpret_cast<const float4 *>(x0) + j);
+        reinterpret_cast<float4 *>(b)[j] = __ldg(reinterpret_cast<const float4 *>(x1) + j);
+      }
+    } else {
+#pragma unroll
+      for (int j = 0; j < DS; ++j) {
+        a[j] = __ldg(x0 + j);
+        b[j] = __ldg(x1 + j);
+      }
+    }
+    float best0 = 3.402823466e38f, best1 = best0;
+    uint32_t c0 = 0, c1 = 0;
+    for (uint32_t c = 0; c < pairs; ++c) {
+      float2 s0 = make_float2(0.0f, 0.0f), s1 = s0;
+#pragma unroll
+      for (int j = 0; j < DS; ++j) {
+        const float2 cv = cs[c * DS + j];
+        const float2 t0 = __ffma2_rn(cv, neg1, make_float2(a[j], a[j]));  // x - c, one rounding
+        const float2 t1 = __ffma2_rn(cv, neg1, make_float2(b[j], b[j]));
+        s0 = __fadd2_rn(s0, __fmul2_rn(t0, t0));
+        s1 = __fadd2_rn(s1, __fmul2_rn(t1, t1));
+      }
+      if (s0.x < best0) { best0 = s0.x; c0 = 2 * c; }
+      if (s0.y < best0) { best0 = s0.y; c0 = 2 * c + 1; }
+      if (s1.x < best1) { best1 = s1.x; c1 = 2 * c; }
+      if (s1.y < best1) { best1 = s1.y; c1 = 2 * c + 1; }
+    }
+    codes[i0 * row_step + m * sub_step] = (uint8_t)c0;
+    codes[i1 * row_step + m * sub_step] = (uint8_t)c1;
+  }
+}
+
+// Codes of n rows (rows `stride` floats apart) by the kernel for this width.
+static DgStatus pq_codes(const float *v, uint64_t n, uint32_t stride, uint32_t M, uint32_t K, uint32_t ds,
+                         const float *cb, uint8_t *codes, uint64_t row_step, uint64_t sub_step, cudaStream_t st) {
+  // float4 loads need rows of whole 16-byte blocks
+  const bool wide = ds % 4 != 0 || (stride % 4 == 0 && (reinterpret_cast<uintptr_t>(v) & 15) == 0);
+  const dim3 grid((unsigned)std::min<uint64_t>((n + 511) / 512, 4096), M), block(256);
+  auto fast = [&](auto kern) { kern<<<grid, block, 0, st>>>(v, n, stride, K, cb, codes, row_step, sub_step); };
+  switch (wide ? ds : 0) {
+    case 2: fast(k_pq_nearest<2>); break;
+    case 4: fast(k_pq_nearest<4>); break;
+    case 6: fast(k_pq_nearest<6>); break;
+    case 8: fast(k_pq_nearest<8>); break;
+    case 10: fast(k_pq_nearest<10>); break;
+    case 12: fast(k_pq_nearest<12>); break;
+    case 16: fast(k_pq_nearest<16>); break;
+    default:
+      k_pq_encode<<<dim3((unsigned)std::min<uint64_t>((n + 127) / 128, 4096), M), 128, 0, st>>>(
+          v, n, stride, M, K, ds, cb, codes, row_step, sub_step);
+  }
+  DG_CUDA(cudaGetLastError());
+  return DG_OK;
 }
 
 // RaBitQ encode_with (src/rabitq.rs:136-149,240-256), one warp per vector.
@@ -277,10 +363,7 @@ DgStatus int8_norms_device(const uint8_t *codes, uint64_t n, uint32_t stride, ui
 DgStatus encode_pq_device(const float *vec, uint64_t n, uint32_t d, uint32_t dpad, uint32_t M,
                           uint32_t K, const float *cb, uint8_t *codes, uint32_t stride,
                           cudaStream_t st) {
-  dim3 grid((unsigned)std::min<uint64_t>((n + 127) / 128, 4096), M);
-  k_pq_encode<<<grid, 128, 0, st>>>(vec, n, dpad, M, K, d / M, cb, codes, stride);
-  DG_CUDA(cudaGetLastError());
-  return DG_OK;
+  return pq_codes(vec, n, dpad, M, K, d / M, cb, codes, stride, 1, st);
 }
 DgStatus encode_rabitq_device(const float *vec, uint64_t n, uint32_t d, uint32_t dpad, uint32_t P,
                               const float *centroid, const float *signs, uint8_t *codes,
@@ -683,87 +766,197 @@ static DgStatus knn_tiled(const float *v, uint64_t n, uint32_t dim, uint32_t dpa
 // ------------------------------------------------------------ PQ training
 // ProductQuantizer::train (src/pq.rs:51-119): per subspace, k-means++ seeding
 // then Lloyd iterations; empty clusters restart from a random training point.
-__global__ void k_mindist_update(const float *S, uint32_t ns, uint32_t d, uint32_t M, uint32_t ds,
-                                 const float *cb, uint32_t K, uint32_t c_new, float *mind) {
-  const uint32_t m = blockIdx.y;
-  const float *cen = cb + ((size_t)m * K + c_new) * ds;
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < ns; i += gridDim.x * blockDim.x) {
+// One seeding step of every subspace (grid.y): distances to the newest seed
+// lower mind (the first step, c_new = 1, starts it), and the last block of a
+// subspace to finish draws seed c_new with probability proportional to mind:
+// the first point whose running sum of mind (FP64) reaches u * total.  A block
+// covers kSeedPts points; its partial sums let the last block find the drawn
+// point in two scans.  One launch per seed; before, an update kernel and a
+// 1024-thread pick whose thread 0 added the partial sums one by one took
+// 31 + 61 us for 50k points x 16 subspaces.
+constexpr int kSeedPts = 1024;
+
+// Inclusive running sums over the 256 threads of a block (s: 8 doubles).
+__device__ __forceinline__ double block_scan256(double v, double *s) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const double t = __shfl_up_sync(kFull, v, o);
+    if (lane >= o) v += t;
+  }
+  __syncthreads();  // s may still be read from the previous scan
+  if (lane == 31) s[warp] = v;
+  __syncthreads();
+  double before = 0.0;
+  for (int w = 0; w < warp; ++w) before += s[w];
+  return before + v;
+}
+
+__global__ void __launch_bounds__(256) k_seed_step(const float *__restrict__ S, uint32_t ns, uint32_t d, uint32_t ds,
+                                                   float *cb, uint32_t K, uint32_t c_new, float *mind, double *part,
+                                                   unsigned int *done, uint64_t seed) {
+  __shared__ double scan[8];
+  __shared__ unsigned int s_pick;
+  const uint32_t m = blockIdx.y, nblk = gridDim.x;
+  const float *cen = cb + ((size_t)m * K + c_new - 1) * ds;
+  float *md = mind + (size_t)m * ns;
+  double *pm = part + (size_t)m * nblk;
+  const bool vec = ds % 4 == 0 && d % 4 == 0;
+  double sum = 0.0;
+#pragma unroll
+  for (int u = 0; u < kSeedPts / 256; ++u) {
+    const uint32_t i = blockIdx.x * kSeedPts + u * 256 + threadIdx.x;
+    if (i >= ns) break;
     const float *x = S + (size_t)i * d + m * ds;
     float acc = 0.0f;
-    for (uint32_t j = 0; j < ds; ++j) {
-      float t = __fsub_rn(x[j], cen[j]);
-      acc = __fadd_rn(acc, __fmul_rn(t, t));
-    }
-    float &md = mind[(size_t)m * ns + i];
-    md = fminf(md, acc);
-  }
-}
-// One block per subspace: D^2-weighted draw of the next seed.
-__global__ void k_pick_next(const float *S, uint32_t ns, uint32_t d, uint32_t ds, float *cb, uint32_t K,
-                            uint32_t c_new, const float *mind, uint64_t seed) {
-  __shared__ double part[1024];
-  __shared__ uint32_t chosen;
-  const uint32_t m = blockIdx.x;
-  const float *md = mind + (size_t)m * ns;
-  const uint32_t per = (ns + blockDim.x - 1) / blockDim.x;
-  const uint32_t lo = threadIdx.x * per, hi = min(ns, lo + per);
-  double s = 0.0;
-  for (uint32_t i = lo; i < hi; ++i) s += md[i];
-  part[threadIdx.x] = s;
-  if (threadIdx.x == 0) chosen = ns - 1;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double tot = 0.0;
-    for (uint32_t t = 0; t < blockDim.x; ++t) tot += part[t];
-    const double u = (double)(rand4(seed, 0x6b6d, m, c_new) >> 11) * (1.0 / 9007199254740992.0);
-    if (tot <= 0.0) {
-      chosen = (uint32_t)range_of(rand4(seed, 0x6b6e, m, c_new), ns);
-    } else {
-      const double thr = u * tot;
-      double cum = 0.0;
-      for (uint32_t t = 0; t < blockDim.x; ++t) {
-        if (cum + part[t] >= thr) {
-          const uint32_t a = t * per, b = min(ns, a + per);
-          for (uint32_t i = a; i < b; ++i) {
-            cum += md[i];
-            if (cum >= thr) {
-              chosen = i;
-              break;
-            }
-          }
-          break;
+    if (vec) {
+      for (uint32_t j = 0; j < ds; j += 4) {
+        const float4 xv = __ldg(reinterpret_cast<const float4 *>(x + j));
+        const float xs[4] = {xv.x, xv.y, xv.z, xv.w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const float t = __fsub_rn(xs[e], cen[j + e]);
+          acc = __fadd_rn(acc, __fmul_rn(t, t));
         }
-        cum += part[t];
       }
-    }
-  }
-  __syncthreads();
-  for (uint32_t j = threadIdx.x; j < ds; j += blockDim.x)
-    cb[((size_t)m * K + c_new) * ds + j] = S[(size_t)chosen * d + m * ds + j];
-}
-__global__ void k_assign_accum(const float *S, uint32_t ns, uint32_t d, uint32_t ds, const float *cb,
-                               uint32_t K, double *sums, unsigned int *counts) {
-  const uint32_t m = blockIdx.y;
-  extern __shared__ float cbs[];
-  for (uint32_t e = threadIdx.x; e < K * ds; e += blockDim.x) cbs[e] = cb[(size_t)m * K * ds + e];
-  __syncthreads();
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < ns; i += gridDim.x * blockDim.x) {
-    const float *x = S + (size_t)i * d + m * ds;
-    float best = 3.402823466e38f;
-    uint32_t bc = 0;
-    for (uint32_t c = 0; c < K; ++c) {
-      float acc = 0.0f;
+    } else {
       for (uint32_t j = 0; j < ds; ++j) {
-        float t = __fsub_rn(x[j], cbs[c * ds + j]);
+        const float t = __fsub_rn(x[j], cen[j]);
         acc = __fadd_rn(acc, __fmul_rn(t, t));
       }
-      if (acc < best) {
-        best = acc;
-        bc = c;
+    }
+    const float v = fminf(c_new == 1 ? 3.402823466e38f : md[i], acc);
+    md[i] = v;
+    sum += (double)v;
+  }
+  const double incl = block_scan256(sum, scan);
+  __threadfence();  // this block's mind before its mark
+  if (threadIdx.x == 255) pm[blockIdx.x] = incl;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) s_pick = atomicAdd(done + m, 1u);
+  __syncthreads();
+  if (s_pick != nblk - 1) return;
+  // the last block of the subspace: the total, then the block and the point
+  __threadfence();
+  double tot = 0.0;
+  for (uint32_t b = threadIdx.x; b < nblk; b += 256) tot += __ldcg(pm + b);
+  tot = block_scan256(tot, scan);
+  __syncthreads();
+  if (threadIdx.x == 255) scan[0] = tot;
+  if (threadIdx.x == 0) s_pick = ns - 1;
+  __syncthreads();
+  tot = scan[0];
+  __syncthreads();
+  if (tot <= 0.0) {
+    if (threadIdx.x == 0) s_pick = (uint32_t)range_of(rand4(seed, 0x6b6e, m, c_new), ns);
+  } else {
+    const double u = (double)(rand4(seed, 0x6b6d, m, c_new) >> 11) * (1.0 / 9007199254740992.0);
+    const double thr = u * tot;
+    // running sums over blocks, then over the points of the block that reaches thr
+    double base = 0.0;
+    uint32_t blk = nblk;  // (none: the last point)
+    for (uint32_t b0 = 0; b0 < nblk && blk == nblk; b0 += 256) {
+      const uint32_t b = b0 + threadIdx.x;
+      const double v = b < nblk ? __ldcg(pm + b) : 0.0;
+      const double c = base + block_scan256(v, scan);
+      __shared__ uint32_t s_first;
+      __shared__ double s_base;
+      if (threadIdx.x == 0) s_first = 0xffffffffu;
+      __syncthreads();
+      if (b < nblk && c >= thr) atomicMin(&s_first, b);
+      __syncthreads();
+      if (s_first != 0xffffffffu ? b == s_first : threadIdx.x == 255) s_base = s_first != 0xffffffffu ? c - v : c;
+      __syncthreads();
+      base = s_base;
+      if (s_first != 0xffffffffu) blk = s_first;
+      __syncthreads();
+    }
+    if (blk < nblk) {
+      if (threadIdx.x == 0) s_pick = min(ns, (blk + 1) * (uint32_t)kSeedPts) - 1;
+      __syncthreads();
+      double v[kSeedPts / 256], s4 = 0.0;
+#pragma unroll
+      for (int e = 0; e < kSeedPts / 256; ++e) {  // four consecutive points per thread
+        const uint32_t i = blk * kSeedPts + threadIdx.x * (kSeedPts / 256) + e;
+        v[e] = i < ns ? (double)__ldcg(md + i) : 0.0;
+        s4 += v[e];
+      }
+      double c = base + block_scan256(s4, scan) - s4;
+#pragma unroll
+      for (int e = 0; e < kSeedPts / 256; ++e) {
+        const uint32_t i = blk * kSeedPts + threadIdx.x * (kSeedPts / 256) + e;
+        c += v[e];
+        if (i < ns && c >= thr) {
+          atomicMin(&s_pick, i);
+          break;
+        }
       }
     }
-    atomicAdd(counts + (size_t)m * K + bc, 1u);
-    for (uint32_t j = 0; j < ds; ++j) atomicAdd(sums + ((size_t)m * K + bc) * ds + j, (double)x[j]);
+  }
+  __syncthreads();
+  const uint32_t chosen = s_pick;
+  for (uint32_t j = threadIdx.x; j < ds; j += 256)
+    cb[((size_t)m * K + c_new) * ds + j] = S[(size_t)chosen * d + m * ds + j];
+  if (threadIdx.x == 0) done[m] = 0u;
+}
+
+// Sums and counts of the points of each cluster (codes: [M][ns]).  A block
+// sorts the numbers of kAccPts points of one subspace by code in shared memory
+// (counting sort), then a warp adds up one cluster's points, lanes over points
+// and coordinates, so that each block adds to a cluster's sums once.  Adding
+// every point's coordinates to global memory took 6.4 ms per iteration for 50k
+// points x 16 subspaces x 8 (FP64 atomics on 2048 addresses per subspace).
+constexpr int kAccPts = 2048;
+__global__ void __launch_bounds__(256) k_cluster_sums(const float *__restrict__ S, uint32_t ns, uint32_t d,
+                                                      uint32_t ds, uint32_t K, const uint8_t *__restrict__ codes,
+                                                      double *sums, unsigned int *counts) {
+  __shared__ uint32_t start[257], fill[256];
+  __shared__ uint16_t order[kAccPts];
+  const uint32_t m = blockIdx.y, p0 = blockIdx.x * kAccPts, np = min((uint32_t)kAccPts, ns - p0);
+  const uint8_t *cm = codes + (size_t)m * ns + p0;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  fill[threadIdx.x] = 0u;
+  __syncthreads();
+  for (uint32_t i = threadIdx.x; i < np; i += 256) atomicAdd(fill + cm[i], 1u);
+  __syncthreads();
+  if (warp == 0) {  // exclusive prefix of the 256 counts, eight per lane
+    uint32_t c[8], sum = 0;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      c[e] = sum;
+      sum += fill[8 * lane + e];
+    }
+    uint32_t incl = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t t = __shfl_up_sync(kFull, incl, o);
+      if (lane >= o) incl += t;
+    }
+#pragma unroll
+    for (int e = 0; e < 8; ++e) start[8 * lane + e] = incl - sum + c[e];
+    if (lane == 31) start[256] = incl;
+  }
+  __syncthreads();
+  fill[threadIdx.x] = start[threadIdx.x];
+  __syncthreads();
+  for (uint32_t i = threadIdx.x; i < np; i += 256) order[atomicAdd(fill + cm[i], 1u)] = (uint16_t)i;
+  __syncthreads();
+  // lanes: `w` coordinates (a power of two) x 32 / w points
+  uint32_t w = 1;
+  while (w < ds && w < 32) w <<= 1;
+  const uint32_t jl = lane & (w - 1), pl = lane / w, pn = 32 / w;
+  for (uint32_t c = warp; c < K; c += 8) {
+    const uint32_t b = start[c], e = start[c + 1];
+    if (b == e) continue;
+    for (uint32_t j0 = 0; j0 < ds; j0 += w) {
+      double acc = 0.0;
+      if (j0 + jl < ds)
+        for (uint32_t i = b + pl; i < e; i += pn) acc += (double)__ldg(S + (size_t)(p0 + order[i]) * d + m * ds + j0 + jl);
+      for (uint32_t o = w; o < 32; o <<= 1) acc += __shfl_xor_sync(kFull, acc, o);
+      if (pl == 0 && j0 + jl < ds) atomicAdd(sums + ((size_t)m * K + c) * ds + j0 + jl, acc);
+    }
+    if (lane == 0) atomicAdd(counts + (size_t)m * K + c, e - b);
   }
 }
 __global__ void k_update(const float *S, uint32_t ns, uint32_t d, uint32_t M, uint32_t ds, float *cb,
@@ -930,20 +1123,24 @@ DgStatus dg_pq_train(const float *X, uint64_t n, uint32_t dim, uint32_t M, uint3
   cudaStream_t st;
   DG_CUDA(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
   float *S = nullptr, *cb = nullptr, *mind = nullptr;
-  double *sums = nullptr;
-  unsigned int *counts = nullptr;
+  double *sums = nullptr, *part = nullptr;
+  unsigned int *counts = nullptr, *done = nullptr;
+  uint8_t *codes = nullptr;
   DgStatus s = DG_OK;
   const size_t cbn = (size_t)M * K * ds;
+  const uint32_t nblk = (ns + kSeedPts - 1) / kSeedPts;
   if (cudaMallocAsync(&S, hs.size() * 4, st) != cudaSuccess || cudaMallocAsync(&cb, cbn * 4, st) != cudaSuccess ||
       cudaMallocAsync(&mind, (size_t)M * ns * 4, st) != cudaSuccess ||
       cudaMallocAsync(&sums, cbn * 8, st) != cudaSuccess ||
-      cudaMallocAsync(&counts, (size_t)M * K * 4, st) != cudaSuccess)
+      cudaMallocAsync(&counts, (size_t)M * K * 4, st) != cudaSuccess ||
+      cudaMallocAsync(&part, (size_t)M * nblk * 8, st) != cudaSuccess ||
+      cudaMallocAsync(&done, (size_t)M * 4, st) != cudaSuccess ||
+      cudaMallocAsync(&codes, (size_t)M * ns, st) != cudaSuccess)
     s = fail(DG_ENOMEM, "pq training staging");
   if (s == DG_OK) {
     cudaMemcpyAsync(S, hs.data(), hs.size() * 4, cudaMemcpyHostToDevice, st);
     // k-means++ seeding (src/pq.rs:301-341)
-    std::vector<float> inf((size_t)M * ns, 3.402823466e38f);
-    cudaMemcpyAsync(mind, inf.data(), inf.size() * 4, cudaMemcpyHostToDevice, st);
+    cudaMemsetAsync(done, 0, (size_t)M * 4, st);
     const uint32_t keff = std::min<uint32_t>(K, ns);
     std::vector<float> hcb(cbn);
     for (uint32_t m = 0; m < M; ++m) {
@@ -952,11 +1149,8 @@ DgStatus dg_pq_train(const float *X, uint64_t n, uint32_t dim, uint32_t M, uint3
                 hcb.begin() + (size_t)m * K * ds);
     }
     cudaMemcpyAsync(cb, hcb.data(), cbn * 4, cudaMemcpyHostToDevice, st);
-    dim3 g((ns + 255) / 256, M);
-    for (uint32_t c = 1; c < keff; ++c) {
-      k_mindist_update<<<g, 256, 0, st>>>(S, ns, dim, M, ds, cb, K, c - 1, mind);
-      k_pick_next<<<M, 1024, 0, st>>>(S, ns, dim, ds, cb, K, c, mind, seed);
-    }
+    for (uint32_t c = 1; c < keff; ++c)
+      k_seed_step<<<dim3(nblk, M), 256, 0, st>>>(S, ns, dim, ds, cb, K, c, mind, part, done, seed);
     // replicate when K exceeds the sample (src/pq.rs:344-350)
     if (keff < K) {
       cudaMemcpyAsync(hcb.data(), cb, cbn * 4, cudaMemcpyDeviceToHost, st);
@@ -968,13 +1162,11 @@ DgStatus dg_pq_train(const float *X, uint64_t n, uint32_t dim, uint32_t M, uint3
       cudaMemcpyAsync(cb, hcb.data(), cbn * 4, cudaMemcpyHostToDevice, st);
     }
     // Lloyd iterations (src/pq.rs:353-408)
-    const size_t smem = (size_t)K * ds * 4;
-    if (smem > 48 * 1024) cudaFuncSetAttribute(k_assign_accum, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    for (uint32_t it = 0; it < iterations; ++it) {
+    for (uint32_t it = 0; it < iterations && s == DG_OK; ++it) {
       cudaMemsetAsync(sums, 0, cbn * 8, st);
       cudaMemsetAsync(counts, 0, (size_t)M * K * 4, st);
-      dim3 ga((unsigned)std::min<uint32_t>((ns + 255) / 256, 256), M);
-      k_assign_accum<<<ga, 256, smem, st>>>(S, ns, dim, ds, cb, K, sums, counts);
+      s = pq_codes(S, ns, dim, M, K, ds, cb, codes, 1, ns, st);
+      k_cluster_sums<<<dim3((ns + kAccPts - 1) / kAccPts, M), 256, 0, st>>>(S, ns, dim, ds, K, codes, sums, counts);
       k_update<<<(M * K + 255) / 256, 256, 0, st>>>(S, ns, dim, M, ds, cb, K, sums, counts, seed, it);
     }
     if (cudaMemcpyAsync(out_codebooks, cb, cbn * 4, cudaMemcpyDeviceToHost, st) != cudaSuccess)
@@ -986,6 +1178,9 @@ DgStatus dg_pq_train(const float *X, uint64_t n, uint32_t dim, uint32_t M, uint3
   if (mind) cudaFreeAsync(mind, st);
   if (sums) cudaFreeAsync(sums, st);
   if (counts) cudaFreeAsync(counts, st);
+  if (part) cudaFreeAsync(part, st);
+  if (done) cudaFreeAsync(done, st);
+  if (codes) cudaFreeAsync(codes, st);
   cudaStreamSynchronize(st);
   cudaStreamDestroy(st);
   return s;

@@ -33,3 +33,19 @@ def test_exact_knn_cosine_against_float64():
     D = 1.0 - Qd @ Xd.T / (np.linalg.norm(Qd, axis=1)[:, None] * np.linalg.norm(Xd, axis=1)[None])
     # the FP64 value rounded to FP32, and the FP64 sums' own rounding of up to 72 terms
     assert np.abs(gd - np.sort(D, axis=1)[:, :10]).max() <= 2.0 ** -24 + 72 * 2.0 ** -50
+
+
+@pytest.mark.parametrize("ds", [1, 2, 3, 4, 6, 8, 10, 12, 16, 20])
+@pytest.mark.parametrize("K", [1, 7, 256])
+def test_pq_encode_widths(oracle, ds, K):
+    M = 3
+    X = synth.mixture(1500, M * ds, 8, seed=4)
+    cb = synth.mixture(M * K, ds, 8, seed=5).reshape(M, K, ds)
+    assert np.array_equal(dg.pq_encode(X, cb), oracle.pq_encode(X, cb))
+
+
+@pytest.mark.parametrize("n,ds,K", [(40, 4, 64), (1025, 8, 32), (5000, 3, 256), (2600, 40, 16)])
+def test_pq_train_blocks(oracle, n, ds, K):
+    X = synth.mixture(n, 2 * ds, 8, seed=6)
+    got = dg.pq_train(X, 2, K, 4, 50_000, seed=9)
+    assert np.array_equal(got, oracle.pq_train(X, 2, K, 4, 50_000, seed=9))

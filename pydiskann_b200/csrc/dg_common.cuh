@@ -83,6 +83,15 @@ __device__ __forceinline__ uint64_t warp_sort_keys(uint64_t key, int lane) {
   return key;
 }
 
+// 16-byte asynchronous copies to shared memory (`bytes` < 16: the rest is zero).
+__device__ __forceinline__ void cp_async16(void *dst, const void *src, uint32_t bytes) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)),
+               "l"(src), "r"(bytes));
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N)); }
+
 // Sum across the LPR lanes of each lane group, transposed: p[i] on entry is
 // this lane's partial for item i (i < LPR); on exit lane r of a group holds
 // the group total of item r.

@@ -1190,15 +1190,6 @@ constexpr int kFrTiles = 16;       // tiles per block of k_route_tcm
 constexpr int kFrCap = 256;        // candidate list of a query (k_fr_select)
 constexpr float kFrEps = 4e-4f;
 
-__device__ __forceinline__ void cp_async16(void *dst, const void *src, uint32_t bytes) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)),
-               "l"(src), "r"(bytes));
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N)); }
-
-
 // The power-of-two scale that brings a vector whose largest |coordinate| is
 // mx below 2^14 (1 for a zero vector), and its inverse.
 __device__ __forceinline__ float2 fr_scale(float mx) {

@@ -17,10 +17,12 @@
 #include <cub/cub.cuh>
 
 #include <algorithm>
+#include <cmath>
+#include <cstring>
 #include <vector>
 
 #include "dg_index.h"
-#include "dg_search.cuh"
+#include "dg_search_cta.cuh"
 
 namespace dg {
 
@@ -64,6 +66,7 @@ struct BuildArgs {
   int32_t metric;
   const float *vf;      // [n][dpad]
   const uint16_t *vb;   // [n][dpad] bf16 (only when every value is bf16-exact)
+  const float *vbn;     // [n] squared norms of the bf16 rows (tensor-core distances)
   const uint32_t *graph;  // snapshot [n][R]
   uint32_t hbits, hB;     // visited table: log2 words, id bits
   uint64_t u0, u1;        // node range of this chunk
@@ -72,35 +75,79 @@ struct BuildArgs {
   uint32_t *cand_cnt;     // [(u1-u0)]
 };
 
-template <int ELEM, int MET, int LPR>
-__device__ __forceinline__ float build_dist(const BuildArgs &a, const float *qs, uint32_t cand, int cnt,
-                                            int lane) {
-  if (ELEM == 1)
-    return rows_distance<LPR, 1, MET>(reinterpret_cast<const uint8_t *>(a.vb), a.dpad * 2,
-                                      (a.dpad / 8) / LPR, qs, cand, cnt, lane, a.metric == DG_L2, 0.0f);
-  return rows_distance<LPR, 0, MET>(reinterpret_cast<const uint8_t *>(a.vf), a.dpad * 4,
-                                    (a.dpad / 4) / LPR, qs, cand, cnt, lane, a.metric == DG_L2, 0.0f);
+// Distances of a warp's cnt <= 32 candidates to the node's own row (qs).  TC:
+// integer-valued rows whose sums are exact in any order, x.q on the tensor
+// cores (the query is its own high half, hi; the low half is zero) and
+// |x|^2 + |q|^2 - 2 x.q in integers.
+template <int ELEM, int MET, int LPR, bool TC>
+__device__ __forceinline__ float build_dist(const BuildArgs &a, const float *qs, const uint16_t *hi, float qq,
+                                            uint32_t cand, int cnt, int lane) {
+  if constexpr (TC) {
+    const float xx = MET == MET_L2 && lane < cnt ? __ldg(a.vbn + cand) : 0.0f;
+    const float dot = bf16_dot_mma(a.vb, a.dpad, hi, cand, cnt, lane);
+    const float v = MET == MET_L2 ? (float)((int)xx + (int)qq - 2 * (int)dot) : dot;
+    return finish_metric(MET, a.metric == DG_L2, v, 0.0f, 0.0f);
+  } else if constexpr (ELEM == 1) {
+    return rows_distance<LPR, 1, MET>(reinterpret_cast<const uint8_t *>(a.vb), a.dpad * 2, (a.dpad / 8) / LPR, qs,
+                                      cand, cnt, lane, a.metric == DG_L2, qq);
+  } else {
+    return rows_distance<LPR, 0, MET>(reinterpret_cast<const uint8_t *>(a.vf), a.dpad * 4, (a.dpad / 4) / LPR, qs,
+                                      cand, cnt, lane, a.metric == DG_L2, qq);
+  }
 }
 
-// Squared norm for the angular metric is recomputed per row inside
-// rows_distance; the query norm is passed through qq.
-template <int ELEM, int MET, int LPR, int LCAP>
-__global__ void __launch_bounds__(128) k_build_search(BuildArgs a, WarpLayout Ly) {
+// Shared memory of one warp's searches: list, new keys, staged candidates,
+// visited table, the node's row (f32, and its BF16 halves), bitmap and count.
+struct BuildLayout {
+  uint32_t list, surv, stage, hash, qf, hi, ctl, total;
+};
+static BuildLayout build_layout(uint32_t Lb, uint32_t R, uint32_t hbits, uint32_t dpad, bool tc) {
+  BuildLayout L{};
+  uint32_t o = 0;
+  L.list = o; o += align16(std::max(Lb, 2u) * 8);
+  L.surv = o; o += cta_surv_bytes(32);
+  L.stage = o; o += align16(R * 4);
+  L.hash = o; o += (1u << hbits) * 4;
+  L.qf = o; o += dpad * 4;
+  L.hi = o; o += tc ? dpad * 4 : 0;
+  L.ctl = o; o += (32 + 4) * 4;
+  L.total = align16(o);
+  return L;
+}
+
+// One warp per node: its current neighbours with their distances, then three
+// greedy searches, each on a list merged in place (cta_merge, one warp).
+// 25k nodes x 128, R = 64, beam 128: 24 ms per pass with a second copy of the
+// list, entry-by-entry merges and FMA distances.
+template <int ELEM, int MET, int LPR, bool TC>
+__global__ void __launch_bounds__(128, 5) k_build_search(BuildArgs a, BuildLayout Ly) {
   extern __shared__ __align__(16) uint8_t smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   uint8_t *wsm = smem + (size_t)warp * Ly.total;
-  uint64_t *W[2] = {reinterpret_cast<uint64_t *>(wsm + Ly.w0), reinterpret_cast<uint64_t *>(wsm + Ly.w1)};
-  uint64_t *cst = reinterpret_cast<uint64_t *>(wsm + Ly.cstage);
+  uint64_t *W = reinterpret_cast<uint64_t *>(wsm + Ly.list);
   uint32_t *stage = reinterpret_cast<uint32_t *>(wsm + Ly.stage);
   const Visited vt{reinterpret_cast<uint32_t *>(wsm + Ly.hash), a.hbits, a.hB};
   float *qs = reinterpret_cast<float *>(wsm + Ly.qf);
+  uint16_t *hi = reinterpret_cast<uint16_t *>(wsm + Ly.hi);
+  uint32_t *map = reinterpret_cast<uint32_t *>(wsm + Ly.ctl), *cnt_s = map + 32;
+  CtaList lists[2];
+  lists[0] = CtaList{W, 0, (int)a.Lb, reinterpret_cast<uint64_t *>(wsm + Ly.surv),
+                     reinterpret_cast<uint16_t *>(wsm + Ly.surv + align16(32 * 8)), map};
+  map[lane] = 0u;
+  if (lane == 0) *cnt_s = 0u;
   const uint64_t gw = blockIdx.x * (uint64_t)(blockDim.x >> 5) + warp;
   const uint64_t nw = (uint64_t)gridDim.x * (blockDim.x >> 5);
   for (uint64_t u = a.u0 + gw; u < a.u1; u += nw) {
     uint64_t *out = a.cand + (u - a.u0) * a.cw;
-    for (uint32_t i = lane; i < a.dpad; i += 32) qs[i] = a.vf[u * a.dpad + i];
+    for (uint32_t i = lane; i < a.dpad; i += 32) {
+      qs[i] = a.vf[u * a.dpad + i];
+      if (TC) {
+        hi[i] = a.vb[u * a.dpad + i];
+        hi[a.dpad + i] = 0;
+      }
+    }
     __syncwarp();
-    float qq = 0.0f;
+    float qq = TC && MET == MET_L2 ? __ldg(a.vbn + u) : 0.0f;
     if (MET == MET_COS) {
       for (uint32_t i = lane; i < a.dpad; i += 32) qq = fmaf(qs[i], qs[i], qq);
 #pragma unroll
@@ -120,10 +167,7 @@ __global__ void __launch_bounds__(128) k_build_search(BuildArgs a, WarpLayout Ly
         if (ok) stage[__popc(m & ((1u << lane) - 1u))] = nb;
         __syncwarp();
         const uint32_t c = lane < cnt ? stage[lane] : 0u;
-        float dd = rows_distance<LPR, ELEM == 1 ? 1 : 0, MET>(
-            ELEM == 1 ? reinterpret_cast<const uint8_t *>(a.vb) : reinterpret_cast<const uint8_t *>(a.vf),
-            ELEM == 1 ? a.dpad * 2 : a.dpad * 4, ELEM == 1 ? (a.dpad / 8) / LPR : (a.dpad / 4) / LPR, qs,
-            c, cnt, lane, a.metric == DG_L2, qq);
+        const float dd = build_dist<ELEM, MET, LPR, TC>(a, qs, hi, qq, c, cnt, lane);
         if (lane < cnt) out[nout + lane] = make_key(dd, c);
         nout += cnt;
         __syncwarp();
@@ -135,40 +179,51 @@ __global__ void __launch_bounds__(128) k_build_search(BuildArgs a, WarpLayout Ly
     for (int s = 0; s < 3; ++s) {
       vt.clear(lane);
       __syncwarp();
-      int cur = 0, wsize = 1;
-      {
-        const uint32_t c = seeds[s];
-        float dd = rows_distance<LPR, ELEM == 1 ? 1 : 0, MET>(
-            ELEM == 1 ? reinterpret_cast<const uint8_t *>(a.vb) : reinterpret_cast<const uint8_t *>(a.vf),
-            ELEM == 1 ? a.dpad * 2 : a.dpad * 4, ELEM == 1 ? (a.dpad / 8) / LPR : (a.dpad / 4) / LPR, qs,
-            c, 1, lane, a.metric == DG_L2, qq);
-        dd = __shfl_sync(kFull, dd, 0);
-        if (lane == 0) {
-          W[0][0] = make_key(dd, c);
-          vt.test_and_set(c);
-        }
-        __syncwarp();
+      int &wsize = lists[0].size, next = 0, ns = 1;
+      wsize = 0;
+      if (lane == 0) {
+        stage[0] = seeds[s];
+        vt.test_and_set(seeds[s]);
       }
+      __syncwarp();
       while (true) {
+        for (int g0 = 0; g0 < ns; g0 += 32) {
+          const int cnt = min(32, ns - g0);
+          const uint32_t c = lane < cnt ? stage[g0 + lane] : DG_PAD;
+          const float dd = build_dist<ELEM, MET, LPR, TC>(a, qs, hi, qq, c, cnt, lane);
+          const uint64_t key = lane < cnt ? make_key(dd, c) : kKeyInvalid;
+          const uint64_t thr = wsize >= (int)a.Lb ? strip_flag(W[a.Lb - 1]) : kKeyInvalid;
+          cta_survive<1>(lists[0], key, key < thr, cnt_s, lane);
+          __syncwarp();
+          const int nk[2] = {(int)*cnt_s, 0};
+          if (nk[0] > 0) {
+            cta_merge<1, 1>(lists, nk, lane, next);
+            if (lane == 0) *cnt_s = 0u;
+            __syncwarp();
+          }
+        }
         int idx = -1;
-        for (int base = 0; base < wsize; base += 32) {
+        for (int base = next; base < wsize; base += 32) {
           const int i = base + lane;
-          const bool un = i < wsize && !key_expanded(W[cur][i]);
-          const uint32_t m = __ballot_sync(kFull, un);
+          const uint32_t m = __ballot_sync(kFull, i < wsize && !key_expanded(W[i]));
           if (m) {
             idx = base + __ffs(m) - 1;
             break;
           }
         }
         if (idx < 0) break;
-        const uint64_t best = W[cur][idx];
-        if (wsize >= (int)a.Lb && key_dist(best) >= key_dist(W[cur][a.Lb - 1])) break;
-        if (lane == 0) W[cur][idx] = best | 1ull;
+        const uint64_t best = W[idx];
+        if (wsize >= (int)a.Lb && key_dist(best) >= key_dist(W[a.Lb - 1])) break;
+        __syncwarp();
+        if (lane == 0) W[idx] = best | 1ull;
+        next = idx + 1;
         const uint32_t *row = a.graph + (size_t)key_id(best) * a.R;
-        int ns = 0;
+        const uint32_t n0 = (uint32_t)lane < a.R ? __ldg(row + lane) : DG_PAD;
+        const uint32_t n1 = (uint32_t)lane + 32 < a.R ? __ldg(row + lane + 32) : DG_PAD;
+        ns = 0;
         for (uint32_t j0 = 0; j0 < a.R; j0 += 32) {
           const uint32_t j = j0 + lane;
-          const uint32_t nb = j < a.R ? __ldg(row + j) : DG_PAD;
+          const uint32_t nb = j0 == 0 ? n0 : j0 == 32 ? n1 : (j < a.R ? __ldg(row + j) : DG_PAD);
           bool ok = nb != DG_PAD && nb < a.n;
           if (ok) ok = !vt.test_and_set(nb);
           const uint32_t m = __ballot_sync(kFull, ok);
@@ -176,18 +231,8 @@ __global__ void __launch_bounds__(128) k_build_search(BuildArgs a, WarpLayout Ly
           ns += __popc(m);
         }
         __syncwarp();
-        for (int g0 = 0; g0 < ns; g0 += 32) {
-          const int cnt = min(32, ns - g0);
-          const uint32_t c = lane < cnt ? stage[g0 + lane] : DG_PAD;
-          const float dd = rows_distance<LPR, ELEM == 1 ? 1 : 0, MET>(
-              ELEM == 1 ? reinterpret_cast<const uint8_t *>(a.vb) : reinterpret_cast<const uint8_t *>(a.vf),
-              ELEM == 1 ? a.dpad * 2 : a.dpad * 4, ELEM == 1 ? (a.dpad / 8) / LPR : (a.dpad / 4) / LPR,
-              qs, c, cnt, lane, a.metric == DG_L2, qq);
-          const uint64_t key = lane < cnt ? make_key(dd, c) : kKeyInvalid;
-          insert_batch(key, W, cur, wsize, (int)a.Lb, cst, lane);
-        }
       }
-      for (int i = lane; i < wsize; i += 32) out[nout + i] = strip_flag(W[cur][i]);
+      for (int i = lane; i < wsize; i += 32) out[nout + i] = strip_flag(W[i]);
       nout += wsize;
       __syncwarp();
     }
@@ -212,6 +257,7 @@ struct PruneArgs {
   int32_t metric;
   uint32_t tile_rows;
   uint32_t *out;            // [n][R]
+  uint32_t skip;            // k_prune: pools of up to this many entries are k_prune_small's
 };
 
 // Distance between candidate rows j and i (rows staged in `tile` when < tile_rows).
@@ -277,6 +323,7 @@ __global__ void __launch_bounds__(kPruneThreads) k_prune(PruneArgs a) {
     const uint64_t u = a.u0 + b;
     const uint64_t off = a.off ? a.off[b] : b * a.stride;
     const uint32_t c = a.cnt[b];
+    if (c <= a.skip) continue;
     const uint64_t *src = a.keys + off;
     // sort the pool (self removed) in shared memory, or in global scratch when large
     uint32_t p2 = 1;
@@ -379,6 +426,350 @@ __global__ void __launch_bounds__(kPruneThreads) k_prune(PruneArgs a) {
   }
 }
 
+// ------------------------------------------------- pools of up to 512 entries
+// k_prune for the usual pools.  robust_prune walks the sorted pool and needs,
+// for every entry it keeps, the distances from it to all later entries; one
+// kept entry at a time leaves a chain of 128 FMAs, a division and a barrier
+// per entry (13 ms per pass of 25k nodes x 128).  Here the next eligible
+// entries are taken as a batch, all their distances are computed at once, and
+// the walk through the batch then only compares: an entry that the batch
+// itself occludes is dropped there, as it would have been.
+//   TC (integer-valued rows whose sums stay below 2^24, so that any order of
+//   summation gives the same bits): batches of 16 on the tensor cores, x.y as
+//   BF16 mma with rows and columns read in the same permuted order of
+//   coordinates, |x|^2 + |y|^2 - 2 x.y in integers;
+//   otherwise batches of 4, a thread per later entry with one FMA chain per
+//   batch entry in coordinate order, as pair_dist.
+constexpr int kSmallPool = 512;
+
+template <bool TC>
+constexpr int prune_batch() { return TC ? 16 : 4; }
+
+// Row stride of the staged rows in 16-byte units: 4 modulo 8 (TC: the four
+// chunks of two rows that a quarter warp reads fall in distinct banks), or odd
+// (a row per lane).
+__host__ __device__ inline uint32_t prune_stride16(uint32_t chunks, bool tc) {
+  return tc ? chunks + ((12u - (chunks & 7u)) & 7u) : chunks | 1u;
+}
+
+// The ratio kd / d of an occlusion test.  It is only ever compared with alpha
+// and with the walk's thresholds 1, 1.2, 1.44, ... up to alpha, so the
+// approximate quotient (2 ulp for |d| in [2^-126, 2^126]) stands in for the
+// rounded one wherever both lie on the same side of each of them; within 8 ulp
+// of one, and for extreme divisors, the rounded quotient is taken.  (The
+// rounded division is a call of some 280 cycles here; it was two thirds of a
+// pruned node's time.)
+__device__ __forceinline__ float prune_ratio(float kd, float d, float alpha) {
+  const float r = __fdividef(kd, d), ad = fabsf(d);
+  bool exact = !(ad > 1e-30f && ad < 1e30f) || fabsf(r - 1.0f) <= 1e-6f || fabsf(r - 1.2f) <= 1.2e-6f ||
+               fabsf(r - alpha) <= 1e-6f * alpha;
+  if (alpha > 1.2f)
+    for (float t = 1.2f; t <= alpha; t = __fmul_rn(t, 1.2f)) exact |= fabsf(r - t) <= 1e-6f * t;
+  if (!exact) return r;
+  return d == 0.0f ? __int_as_float(0x7f800000) : __fdiv_rn(kd, d);
+}
+
+struct PruneSmem {
+  uint64_t ka[kSmallPool], kb[kSmallPool];
+  float occ[kSmallPool];
+  int norm[kSmallPool];
+  float D[16][kSmallPool + 4];  // (padded: the tensor-core stores are conflict-free)
+  uint32_t out[kStageCap];
+  int bi[16];       // the batch: pool positions
+  int nb, cursor;   // its size, where the next one starts
+  uint32_t selected;  // which of the batch stay
+  float ratio[16][17];  // [q][l]: occlusion of batch entry l by entry q < l
+  uint32_t cnt[8];
+  uint8_t sel[kSmallPool];
+};
+
+template <int ELEM, int MET, bool TC>
+__global__ void __launch_bounds__(kPruneThreads, 2) k_prune_small(PruneArgs a) {
+  extern __shared__ __align__(16) uint8_t smem[];
+  PruneSmem &P = *reinterpret_cast<PruneSmem *>(smem);
+  uint4 *tile = reinterpret_cast<uint4 *>(smem + ((sizeof(PruneSmem) + 15) & ~(size_t)15));
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  constexpr int B = prune_batch<TC>();
+  const uint32_t chunks = ELEM == 1 ? a.dpad / 8 : a.dpad / 4, ts = prune_stride16(chunks, TC);
+  const uint8_t *rows = ELEM == 1 ? reinterpret_cast<const uint8_t *>(a.vb) : reinterpret_cast<const uint8_t *>(a.vf);
+  for (uint64_t b = blockIdx.x; b < a.nodes; b += gridDim.x) {
+    const uint64_t u = a.u0 + b;
+    const uint32_t c = a.cnt[b];
+    if (c > (uint32_t)kSmallPool) continue;
+    const uint64_t *src = a.keys + (a.off ? a.off[b] : b * a.stride);
+    // ---- sort (self removed): every warp sorts 64 keys in registers (entries
+    // lane and lane + 32 of its run), then each key's place is its rank in its
+    // own run plus the keys before it in the other runs
+    const uint32_t runs = (c + 63) / 64;
+    uint64_t k0 = kKeyInvalid, k1 = kKeyInvalid;
+    {
+      const uint32_t i0 = 64 * warp + lane, i1 = i0 + 32;
+      if (i0 < c) k0 = strip_flag(src[i0]);
+      if (i1 < c) k1 = strip_flag(src[i1]);
+      if (k0 != kKeyInvalid && key_id(k0) == (uint32_t)u) k0 = kKeyInvalid;
+      if (k1 != kKeyInvalid && key_id(k1) == (uint32_t)u) k1 = kKeyInvalid;
+    }
+    if ((uint32_t)warp < runs) {
+      k0 = warp_sort_keys(k0, lane);
+      k1 = shfl64(warp_sort_keys(k1, lane), 31 - lane);  // descending: k0 then k1 is bitonic
+      if (k1 < k0) {
+        const uint64_t t = k0;
+        k0 = k1;
+        k1 = t;
+      }
+#pragma unroll
+      for (int j = 16; j > 0; j >>= 1) {
+        const uint64_t o0 = shfl_xor64(k0, j), o1 = shfl_xor64(k1, j);
+        const bool low = (lane & j) == 0;
+        k0 = (o0 < k0) == low ? o0 : k0;
+        k1 = (o1 < k1) == low ? o1 : k1;
+      }
+      P.ka[64 * warp + lane] = k0;
+      P.ka[64 * warp + 32 + lane] = k1;
+    }
+    __syncthreads();
+    if ((uint32_t)warp < runs) {
+      int p0 = lane, p1 = lane + 32;
+      for (uint32_t r = 0; r < runs; ++r) {
+        if (r == (uint32_t)warp) continue;
+        const uint64_t *run = P.ka + 64 * r;
+        // keys of run r before mine; equal keys of an earlier run go first
+        const uint64_t b0 = k0 + (r < (uint32_t)warp ? 1u : 0u), b1 = k1 + (r < (uint32_t)warp ? 1u : 0u);
+        int q0 = 0, q1 = 0;
+#pragma unroll
+        for (int step = 32; step > 0; step >>= 1) {
+          q0 += run[q0 + step - 1] < b0 ? step : 0;
+          q1 += run[q1 + step - 1] < b1 ? step : 0;
+        }
+        p0 += q0 + (q0 == 63 && run[63] < b0);
+        p1 += q1 + (q1 == 63 && run[63] < b1);
+      }
+      if (k0 != kKeyInvalid) P.kb[p0] = k0;
+      if (k1 != kKeyInvalid) P.kb[p1] = k1;
+    }
+    // ---- de-duplicate (same id => same key), keeping order: kb[0 .. valid) -> ka
+    const int valid = __syncthreads_count(k0 != kKeyInvalid) + __syncthreads_count(k1 != kKeyInvalid);
+    uint32_t keep[2];
+    uint64_t mine[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int i = 64 * warp + 32 * h + lane;
+      mine[h] = i < valid ? P.kb[i] : kKeyInvalid;
+      keep[h] = __ballot_sync(kFull, i < valid && (i == 0 || P.kb[i - 1] != mine[h]));
+    }
+    if (lane == 0) P.cnt[warp] = __popc(keep[0]) + __popc(keep[1]);
+    __syncthreads();
+    int before = 0, m = 0;
+    for (int w = 0; w < 8; ++w) {
+      before += w < warp ? (int)P.cnt[w] : 0;
+      m += (int)P.cnt[w];
+    }
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      if ((keep[h] >> lane) & 1u) P.ka[before + (h ? __popc(keep[0]) : 0) + __popc(keep[h] & lanemask_lt(lane))] = mine[h];
+    }
+    const uint64_t *K = P.ka;
+    for (int i = tid; i < m; i += kPruneThreads) {
+      P.occ[i] = 0.0f;
+      P.sel[i] = 0;
+    }
+    __syncthreads();
+    // ---- stage rows (and, TC, their squared norms)
+    const int staged = min(m, (int)a.tile_rows);
+#pragma unroll 8
+    for (uint32_t e = tid; e < staged * chunks; e += kPruneThreads) {
+      const uint32_t r = e / chunks, t = e - r * chunks;
+      cp_async16(tile + r * ts + t, reinterpret_cast<const uint4 *>(rows) + (size_t)key_id(K[r]) * chunks + t, 16);
+    }
+    cp_async_commit();
+    cp_async_wait<0>();
+    __syncthreads();
+    auto row_of = [&](int j) -> const uint4 * {
+      return j < staged ? tile + (size_t)j * ts : reinterpret_cast<const uint4 *>(rows) + (size_t)key_id(K[j]) * chunks;
+    };
+    if (TC) {
+      for (int j = 8 * warp + (lane >> 2); j < m; j += 64) {  // four lanes per row
+        const uint4 *x = row_of(j);
+        float s2 = 0.0f;
+        for (uint32_t t = lane & 3; t < chunks; t += 4) {
+          float v[8];
+          Chunk<1>::unpack(x[t], v);
+#pragma unroll
+          for (int e = 0; e < 8; ++e) s2 = fmaf(v[e], v[e], s2);
+        }
+        s2 += __shfl_xor_sync(__activemask(), s2, 1);
+        s2 += __shfl_xor_sync(__activemask(), s2, 2);
+        if ((lane & 3) == 0) P.norm[j] = (int)s2;
+      }
+    }
+    // ---- robust_prune (src/lib.rs:977-1034)
+    const float alpha = fmaxf(a.alpha, 1.0f);
+    float cur_alpha = 1.0f;
+    uint32_t np = 0;
+    while (cur_alpha <= alpha && np < a.R) {
+      int from = 0;
+      while (np < a.R) {
+        __syncthreads();  // occlusion and selection of the previous batch (and the norms) are in place
+        if (warp == 0) {
+          int nb = 0, at = m;
+          for (int base = from; base < m && nb < B; base += 32) {
+            const int i = base + lane;
+            const bool ok = i < m && !P.sel[i] && P.occ[i] <= cur_alpha;
+            const uint32_t mk = __ballot_sync(kFull, ok);
+            const int rank = nb + __popc(mk & lanemask_lt(lane));
+            if (ok && rank < B) P.bi[rank] = i;
+            const uint32_t last = __ballot_sync(kFull, ok && rank == B - 1);
+            if (last) at = base + __ffs(last);
+            nb = min(B, nb + __popc(mk));
+          }
+          if (lane == 0) {
+            P.nb = nb;
+            P.cursor = at;
+          }
+        }
+        __syncthreads();
+        const int nb = P.nb, next = P.cursor;
+        if (nb == 0) break;
+        const int j0 = P.bi[0] + 1;
+        // ---- distances from the batch to every later entry that can still be kept
+        if (TC) {
+          const int g = lane >> 2, t = lane & 3;
+          const uint4 *col0 = row_of(P.bi[min(g, nb - 1)]), *col1 = row_of(P.bi[min(g + 8, nb - 1)]);
+          const bool wide = nb > 8;
+          int cn[4];  // squared norms of this lane's columns 2t, 2t + 1 (+ 8)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) cn[e] = MET == MET_L2 ? P.norm[P.bi[min(2 * t + (e & 1) + (e >> 1) * 8, nb - 1)]] : 0;
+          for (int jt = (j0 & ~15) + 16 * warp; jt < m; jt += 16 * 8) {
+            const uint4 *r0 = row_of(min(jt + g, m - 1)), *r1 = row_of(min(jt + g + 8, m - 1));
+            float d0[4] = {}, d1[4] = {};
+#pragma unroll 4
+            for (uint32_t ch = t; ch < chunks; ch += 4) {
+              const uint4 x0 = r0[ch], x1 = r1[ch], y0 = col0[ch];
+              mma_bf16_16x8x16(d0, x0.x, x1.x, x0.y, x1.y, y0.x, y0.y);
+              mma_bf16_16x8x16(d0, x0.z, x1.z, x0.w, x1.w, y0.z, y0.w);
+              if (wide) {
+                const uint4 y1 = col1[ch];
+                mma_bf16_16x8x16(d1, x0.x, x1.x, x0.y, x1.y, y1.x, y1.y);
+                mma_bf16_16x8x16(d1, x0.z, x1.z, x0.w, x1.w, y1.z, y1.w);
+              }
+            }
+            // lane (g, t): rows jt + g, jt + g + 8 x columns 2t, 2t + 1 (+ 8)
+            const int rn[2] = {MET == MET_L2 && jt + g < m ? P.norm[jt + g] : 0,
+                               MET == MET_L2 && jt + g + 8 < m ? P.norm[jt + g + 8] : 0};
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+              const int col = 2 * t + (e & 1) + (e >= 4 ? 8 : 0), j = jt + g + ((e & 2) ? 8 : 0);
+              if (col < nb && j < m) {
+                const float dot = e < 4 ? d0[e] : d1[e & 3];
+                float v = dot;
+                if (MET == MET_L2) v = (float)(rn[(e >> 1) & 1] + cn[(e & 1) + (e >> 2) * 2] - 2 * (int)dot);
+                P.D[col][j] = finish_metric(MET, a.metric == DG_L2, v, 0.0f, 0.0f);
+              }
+            }
+          }
+        } else {
+          const uint4 *col[B];
+#pragma unroll
+          for (int q = 0; q < B; ++q) col[q] = row_of(P.bi[min(q, nb - 1)]);
+          for (int j = j0 + tid; j < m; j += kPruneThreads) {
+            if (P.sel[j] || P.occ[j] > alpha) continue;
+            const uint4 *x = row_of(j);
+            constexpr int E = Chunk<ELEM>::EPC;
+            float ab[B], aa = 0.0f, bb[B];
+#pragma unroll
+            for (int q = 0; q < B; ++q) ab[q] = bb[q] = 0.0f;
+            for (uint32_t ch = 0; ch < chunks; ++ch) {
+              float xv[E];
+              Chunk<ELEM>::unpack(x[ch], xv);
+              if (MET == MET_COS) {
+#pragma unroll
+                for (int e = 0; e < E; ++e) aa = fmaf(xv[e], xv[e], aa);
+              }
+#pragma unroll
+              for (int q = 0; q < B; ++q) {
+                float yv[E];
+                Chunk<ELEM>::unpack(col[q][ch], yv);
+#pragma unroll
+                for (int e = 0; e < E; ++e) {
+                  if (MET == MET_L2) {
+                    const float df = xv[e] - yv[e];
+                    ab[q] = fmaf(df, df, ab[q]);
+                  } else {
+                    ab[q] = fmaf(xv[e], yv[e], ab[q]);
+                    if (MET == MET_COS) bb[q] = fmaf(yv[e], yv[e], bb[q]);
+                  }
+                }
+              }
+            }
+#pragma unroll
+            for (int q = 0; q < B; ++q)
+              if (q < nb) P.D[q][j] = finish_metric(MET, a.metric == DG_L2, ab[q], aa, bb[q]);
+          }
+        }
+        __syncthreads();
+        // ---- which of the batch stay: the occlusions inside the batch, a thread
+        // each, then warp 0 walks through them (lane l is entry l)
+        if (tid < B * B) {
+          const int q = tid / B, l = tid % B;
+          if (q < l && l < nb) {
+            const int i = P.bi[l];
+            P.ratio[q][l] = prune_ratio(key_dist(K[i]), P.D[q][i], alpha);
+          }
+        }
+        __syncthreads();
+        if (warp == 0) {
+          const int l = min(lane, nb - 1), iq = P.bi[l];
+          float oq = P.occ[iq], rt[B];
+#pragma unroll
+          for (int q = 0; q < B; ++q) rt[q] = q < l && lane < nb ? P.ratio[q][l] : 0.0f;
+          uint32_t sel = 0, kept = 0;
+#pragma unroll
+          for (int q = 0; q < B; ++q) {
+            if (q < nb && np + kept < a.R && __shfl_sync(kFull, oq, q) <= cur_alpha) {
+              sel |= 1u << q;
+              ++kept;
+              oq = fmaxf(oq, rt[q]);
+            }
+          }
+          if (lane < nb && ((sel >> lane) & 1u)) P.out[np + __popc(sel & lanemask_lt(lane))] = key_id(K[iq]);
+          if (lane == 0) P.selected = sel;
+        }
+        __syncthreads();
+        const uint32_t selected = P.selected, count = __popc(selected);
+        // ---- occlusion of the later entries by the kept ones
+        for (int j = j0 + tid; j < m; j += kPruneThreads) {
+          float o = P.occ[j];
+          if (P.sel[j] || o > alpha) continue;
+          const float kj = key_dist(K[j]);
+#pragma unroll
+          for (int q = 0; q < B; ++q)
+            if (((selected >> q) & 1u) && P.bi[q] < j) o = fmaxf(o, prune_ratio(kj, P.D[q][j], alpha));
+          P.occ[j] = o;
+        }
+        __syncthreads();  // (selection flags are read above)
+        if (warp == 0 && lane < nb && ((selected >> lane) & 1u)) P.sel[P.bi[lane]] = 1;
+        np += count;
+        from = next;
+      }
+      cur_alpha = __fmul_rn(cur_alpha, 1.2f);
+    }
+    __syncthreads();
+    // ---- fill with the nearest entries not kept
+    if (warp == 0) {
+      for (int base = 0; base < m && np < a.R; base += 32) {
+        const int i = base + lane;
+        const bool ok = i < m && !P.sel[i];
+        const uint32_t mk = __ballot_sync(kFull, ok);
+        const uint32_t at = np + __popc(mk & lanemask_lt(lane));
+        if (ok && at < a.R) P.out[at] = key_id(K[i]);
+        np = min(a.R, np + (uint32_t)__popc(mk));
+      }
+      for (uint32_t j = lane; j < a.R; j += 32) a.out[u * a.R + j] = j < np ? P.out[j] : DG_PAD;
+    }
+    __syncthreads();
+  }
+}
+
 // ---------------------------------------------------------- symmetrisation
 __global__ void k_degrees(const uint32_t *g, uint64_t n, uint32_t R, uint32_t *outdeg, uint32_t *indeg) {
   for (uint64_t e = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; e < n * R;
@@ -442,11 +833,26 @@ __global__ void k_pool_keys(const float *vf, const uint16_t *vb, uint64_t n, uin
   }
 }
 
-__global__ void k_bf16_exact(const float *v, uint64_t total, unsigned int *flag) {
+// What the build may assume of the values: out[0] bit 0 set when one is not
+// exact in BF16, bit 1 when one is not an integer; out[1], out[2]: ordered bits
+// of the largest and of the smallest.
+__global__ void k_value_range(const float *v, uint64_t total, uint32_t *out) {
+  uint32_t f = 0, hi = 0, lo = 0xffffffffu;
   for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < total;
        i += (uint64_t)gridDim.x * blockDim.x) {
     const float x = v[i];
-    if (__uint_as_float(__float_as_uint(x) & 0xffff0000u) != x) atomicOr(flag, 1u);
+    f |= __uint_as_float(__float_as_uint(x) & 0xffff0000u) != x ? 1u : 0u;
+    f |= x != rintf(x) ? 2u : 0u;
+    hi = max(hi, ordered_bits(x));
+    lo = min(lo, ordered_bits(x));
+  }
+  f = __reduce_or_sync(kFull, f);
+  hi = __reduce_max_sync(kFull, hi);
+  lo = __reduce_min_sync(kFull, lo);
+  if ((threadIdx.x & 31) == 0) {
+    if (f) atomicOr(out, f);
+    atomicMax(out + 1, hi);
+    atomicMin(out + 2, lo);
   }
 }
 
@@ -457,12 +863,11 @@ static uint32_t id_bits(uint64_t n) {
 }
 
 template <int ELEM, int MET>
-static DgStatus run_build(const BuildArgs &base, float *vf, uint16_t *vb, uint32_t *g0, uint32_t *g1,
+static DgStatus run_build(const BuildArgs &base, float *vf, uint16_t *vb, bool tc, uint32_t *g0, uint32_t *g1,
                           float alpha, cudaStream_t st, uint32_t **result) {
   const uint64_t n = base.n;
   const uint32_t R = base.R, dpad = base.dpad;
   constexpr int LPR = ELEM == 1 ? 4 : 8;
-  const int lcap = base.Lb <= 64 ? 64 : base.Lb <= 256 ? 256 : 1024;
   int dev = 0, sms = 0;
   DG_CUDA(cudaGetDevice(&dev));
   DG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
@@ -483,13 +888,39 @@ static DgStatus run_build(const BuildArgs &base, float *vf, uint16_t *vb, uint32
   int pblocks = 0;
   DG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&pblocks, prune_k, kPruneThreads, psmem));
   const int pgrid = std::max(1, pblocks) * sms;
+  // pools of up to kSmallPool entries: two CTAs per SM, the rest of whose shared
+  // memory stages rows
+  void (*small_k)(PruneArgs) = k_prune_small<ELEM, MET, false>;
+  if constexpr (ELEM == 1 && MET != MET_COS)
+    if (tc) small_k = k_prune_small<ELEM, MET, true>;
+  const uint32_t row16 = prune_stride16(ELEM == 1 ? dpad / 8 : dpad / 4, tc);
+  const size_t fixed = (sizeof(PruneSmem) + 15) & ~(size_t)15;
+  const uint32_t small_rows = (uint32_t)std::min<size_t>(kSmallPool, (112 * 1024 - fixed) / (row16 * 16));
+  const size_t ssmem = fixed + (size_t)small_rows * row16 * 16;
+  DG_CUDA(cudaFuncSetAttribute(small_k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ssmem));
+  auto prune = [&](PruneArgs p, uint64_t nodes, uint64_t largest) -> DgStatus {
+    PruneArgs q = p;
+    q.tile_rows = small_rows;
+    small_k<<<(int)std::min<uint64_t>(2ull * sms, nodes), kPruneThreads, ssmem, st>>>(q);
+    DG_CUDA(cudaGetLastError());
+    if (largest > (uint64_t)kSmallPool) {
+      p.skip = kSmallPool;
+      prune_k<<<(int)std::min<uint64_t>(pgrid, nodes), kPruneThreads, psmem, st>>>(p);
+      DG_CUDA(cudaGetLastError());
+    }
+    return DG_OK;
+  };
   // search kernel geometry
   const uint32_t hbits = base.Lb <= 64 ? 10 : base.Lb <= 128 ? 11 : 12;
-  const WarpLayout Ly = warp_layout(ELEM == 1 ? TRAV_BF16 : TRAV_F32, lcap, false, hbits, dpad, 0, 0, 0);
-  void (*sk)(BuildArgs, WarpLayout) = lcap == 64 ? k_build_search<ELEM, MET, LPR, 64>
-                                    : lcap == 256 ? k_build_search<ELEM, MET, LPR, 256>
-                                                  : k_build_search<ELEM, MET, LPR, 1024>;
-  DG_CUDA(cudaFuncSetAttribute(sk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(Ly.total * 4)));
+  const BuildLayout Ly = build_layout(base.Lb, R, hbits, dpad, tc);
+  void (*sk)(BuildArgs, BuildLayout) = k_build_search<ELEM, MET, LPR, false>;
+  if constexpr (ELEM == 1 && MET != MET_COS)
+    if (tc) sk = k_build_search<ELEM, MET, LPR, true>;
+  // (accepted or refused by the state of a two-list search, as ever)
+  const uint32_t lcap = base.Lb <= 64 ? 64 : base.Lb <= 256 ? 256 : 1024;
+  const WarpLayout limit = warp_layout(ELEM == 1 ? TRAV_BF16 : TRAV_F32, lcap, false, hbits, dpad, 0, 0, 0);
+  DG_CUDA(cudaFuncSetAttribute(sk, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)std::max(limit.total * 4, Ly.total * 4)));
   int sblocks = 0;
   DG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&sblocks, sk, 128, Ly.total * 4));
   if (sblocks < 1) return fail(DG_ENOTSUP, "build search state does not fit in shared memory");
@@ -551,8 +982,8 @@ static DgStatus run_build(const BuildArgs &base, float *vf, uint16_t *vb, uint32
         p.gsort = gsort;
         p.gcap = gcap;
       }
-      k_prune<ELEM, MET><<<(int)std::min<uint64_t>(pgrid, nodes), kPruneThreads, psmem, st>>>(p);
-      DG_CUDA(cudaGetLastError());
+      DgStatus ps = prune(p, nodes, cw);
+      if (ps != DG_OK) return ps;
     }
     // symmetrise: union of outgoing and incoming, distances, prune into `cur`
     DG_CUDA(cudaMemsetAsync(outdeg, 0, n * 4, st));
@@ -603,8 +1034,8 @@ static DgStatus run_build(const BuildArgs &base, float *vf, uint16_t *vb, uint32
       p.gsort = gsort;
       p.gcap = gcap_sym;
     }
-    k_prune<ELEM, MET><<<(int)std::min<uint64_t>(pgrid, n), kPruneThreads, psmem, st>>>(p);
-    DG_CUDA(cudaGetLastError());
+    DgStatus ps = prune(p, n, maxpool);
+    if (ps != DG_OK) return ps;
   }
   DG_CUDA(cudaStreamSynchronize(st));
   cudaFreeAsync(cand, st);
@@ -643,25 +1074,41 @@ extern "C" DgStatus dg_build_vamana(const float *X, uint64_t n, uint32_t dim, in
   float *vf = nullptr;
   uint16_t *vb = nullptr;
   uint32_t *g0 = nullptr, *g1 = nullptr;
-  unsigned int *flag = nullptr;
+  uint32_t *flag = nullptr;
+  float *vbn = nullptr;
   DgStatus s = DG_OK;
   if (cudaMallocAsync(&vf, n * dpad * 4, st) != cudaSuccess || cudaMallocAsync(&g0, n * R * 4, st) != cudaSuccess ||
-      cudaMallocAsync(&g1, n * R * 4, st) != cudaSuccess || cudaMallocAsync(&flag, 4, st) != cudaSuccess)
+      cudaMallocAsync(&g1, n * R * 4, st) != cudaSuccess || cudaMallocAsync(&flag, 12, st) != cudaSuccess)
     s = fail(DG_ENOMEM, "build staging");
   if (s == DG_OK) s = upload_rows_f32(X, n, dim, dpad, vf, st);
-  bool exact_bf16 = false;
+  bool exact_bf16 = false, tc = false;
   if (s == DG_OK) {
     // BF16 rows carry the same values when every coordinate is bf16-exact
     // (integer data in [-256, 256], BF16-stored embeddings): half the gather bytes.
-    cudaMemsetAsync(flag, 0, 4, st);
-    k_bf16_exact<<<148 * 8, 256, 0, st>>>(vf, n * dpad, flag);
-    unsigned int hf = 1;
-    cudaMemcpyAsync(&hf, flag, 4, cudaMemcpyDeviceToHost, st);
+    uint32_t hf[3] = {0u, 0u, 0xffffffffu};
+    cudaMemcpyAsync(flag, hf, 12, cudaMemcpyHostToDevice, st);
+    k_value_range<<<148 * 8, 256, 0, st>>>(vf, n * dpad, flag);
+    hf[0] = 3u;
+    cudaMemcpyAsync(hf, flag, 12, cudaMemcpyDeviceToHost, st);
     cudaStreamSynchronize(st);
-    exact_bf16 = hf == 0 && metric != DG_COSINE;
+    exact_bf16 = !(hf[0] & 1u) && metric != DG_COSINE;
+    // integers whose sums of products and of squared differences stay below
+    // 2^24: every partial sum is exact, so the order of summation is free and
+    // the tensor cores return the FMA chain's bits
+    auto value = [](uint32_t o) {
+      const uint32_t b = (o & 0x80000000u) ? (o & 0x7fffffffu) : ~o;
+      float f;
+      std::memcpy(&f, &b, 4);
+      return (double)f;
+    };
+    const double hi = value(hf[1]), lo = value(hf[2]), mx = std::max(std::fabs(hi), std::fabs(lo));
+    tc = exact_bf16 && !(hf[0] & 2u) && (double)dim * mx * mx < 16777216.0 &&
+         (double)dim * (hi - lo) * (hi - lo) < 16777216.0;
     if (exact_bf16) {
-      if (cudaMallocAsync(&vb, n * dpad * 2, st) != cudaSuccess) s = fail(DG_ENOMEM, "build staging");
-      else s = encode_bf16_device(vf, n, dpad, vb, st);
+      if (cudaMallocAsync(&vb, n * dpad * 2, st) != cudaSuccess || cudaMallocAsync(&vbn, n * 4, st) != cudaSuccess)
+        s = fail(DG_ENOMEM, "build staging");
+      else
+        s = encode_bf16_device(vf, n, dpad, vb, st, tc ? vbn : nullptr);
     }
   }
   if (s == DG_OK) {
@@ -682,14 +1129,15 @@ extern "C" DgStatus dg_build_vamana(const float *X, uint64_t n, uint32_t dim, in
     a.metric = metric;
     a.vf = vf;
     a.vb = vb;
+    a.vbn = vbn;
     const int met = metric == DG_DOT ? MET_DOT : metric == DG_COSINE ? MET_COS : MET_L2;
     if (exact_bf16) {
-      s = met == MET_DOT ? run_build<1, MET_DOT>(a, vf, vb, g0, g1, alpha, st, &result)
-                         : run_build<1, MET_L2>(a, vf, vb, g0, g1, alpha, st, &result);
+      s = met == MET_DOT ? run_build<1, MET_DOT>(a, vf, vb, tc, g0, g1, alpha, st, &result)
+                         : run_build<1, MET_L2>(a, vf, vb, tc, g0, g1, alpha, st, &result);
     } else {
-      s = met == MET_DOT   ? run_build<0, MET_DOT>(a, vf, vb, g0, g1, alpha, st, &result)
-          : met == MET_COS ? run_build<0, MET_COS>(a, vf, vb, g0, g1, alpha, st, &result)
-                           : run_build<0, MET_L2>(a, vf, vb, g0, g1, alpha, st, &result);
+      s = met == MET_DOT   ? run_build<0, MET_DOT>(a, vf, vb, tc, g0, g1, alpha, st, &result)
+          : met == MET_COS ? run_build<0, MET_COS>(a, vf, vb, tc, g0, g1, alpha, st, &result)
+                           : run_build<0, MET_L2>(a, vf, vb, tc, g0, g1, alpha, st, &result);
     }
   }
   if (s == DG_OK) {
@@ -699,6 +1147,7 @@ extern "C" DgStatus dg_build_vamana(const float *X, uint64_t n, uint32_t dim, in
   }
   if (vf) cudaFreeAsync(vf, st);
   if (vb) cudaFreeAsync(vb, st);
+  if (vbn) cudaFreeAsync(vbn, st);
   if (g0) cudaFreeAsync(g0, st);
   if (g1) cudaFreeAsync(g1, st);
   if (flag) cudaFreeAsync(flag, st);

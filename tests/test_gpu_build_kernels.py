@@ -49,3 +49,16 @@ def test_pq_train_blocks(oracle, n, ds, K):
     X = synth.mixture(n, 2 * ds, 8, seed=6)
     got = dg.pq_train(X, 2, K, 4, 50_000, seed=9)
     assert np.array_equal(got, oracle.pq_train(X, 2, K, 4, 50_000, seed=9))
+
+
+@pytest.mark.parametrize("d,centres,sigma,R,Lb", [(33, 4, 20.0, 5, 20), (128, 8, 20.0, 64, 128), (16, 1, 1.0, 24, 40),
+                                                  (257, 4, 20.0, 16, 30), (40, 8, 20.0, 16, 200)])
+@pytest.mark.parametrize("shift", [0.0, 0.5])
+def test_vamana_prune_batches(oracle, d, centres, sigma, R, Lb, shift):
+    """Tensor-core batches (integers whose sums stay below 2^24), FMA batches (halves: not
+    integers, but every sum still exact; 257-d: sums past the bound), pools of repeats (sigma 1)
+    and pools above 512 entries (beam 200): the oracle's graph, edge for edge."""
+    X = synth.mixture(900, d, centres, seed=8, sigma=sigma) + np.float32(shift)
+    adj, med = dg.build_graph(X, R, Lb, 1.2, seed=5)
+    want, _ = oracle.build_vamana(X, R, Lb, 1.2, seed=5, medoid_id=med)
+    assert np.array_equal(adj, want)

@@ -61,6 +61,7 @@ struct DgSpfresh {
   // grouped by posting, work items, per-pair candidate lists
   DgIndex::Buf probe, probe_cnt, pcount, pstart, pfill, istart, pair_q, pos_of, items, pair_keys, pair_cnt, misc;
   DgIndex::Buf qthr;  // posting-major scan: per query, a bound of its k-th distance
+  DgIndex::Buf pm_q;  // posting-major scan: FP16 query rows, norms and largest coordinates
 };
 
 namespace dg {
@@ -878,60 +879,55 @@ __host__ __device__ inline uint32_t pm_ks(uint32_t d) { return ((d + 15u) & ~15u
 // Capacity of a pair's k-best list: k rounded up to 16 (at most kPmK), which
 // keeps the scan's shared memory at three CTAs per SM for d = 96, k <= 16.
 __host__ __device__ inline uint32_t pm_kcap(uint32_t k) { return (k + 15u) & ~15u; }
+// Floats of the tile area: f32 rows of d + 4 floats, or kPmQ x kPmT candidate keys.
+__host__ __device__ inline uint32_t pm_tile_floats(uint32_t d) {
+  const uint32_t rows = (uint32_t)kPmT * (d + 4u), keys = (uint32_t)kPmQ * kPmT * 2u;
+  return rows > keys ? rows : keys;
+}
 
-// One CTA (8 warps) per work item at a time: the item's queries and a tile of
-// the posting's entries in shared memory; warp w scores queries w, w+8, ...
-// against two entries per lane and keeps each query's k best.  The dot
-// products of a tile come from the tensor cores (the warps split the 64 x 32
-// tile into 16 x 16 blocks) when the tile and the queries meet the exactness
-// bounds above, else from an FMA chain per pair.
 // qthr[q] for each query of a posting-major chunk (a warp each): an upper
 // bound of the query's k-th smallest scan distance, from the live entries of
-// its first probe (the nearest one).  B, the k-th smallest of their
-// coordinate-order squared distances, is within (d + 2) 2^-24 B of the exact
-// value; the scan's |q|^2 + |x|^2 - 2 q.x differs from the exact value by at
-// most (2d + 6) 2^-24 (|q|^2 + |x|^2).  So
-//     B (1 + (d + 2) 2^-23) + 4 (d + 4) 2^-24 (|q|^2 + max |x|^2)
+// its first probe (the nearest one).  B, the k-th smallest of their squared
+// distances (FP32 sums of d squares, in any order), is within (d + 2) 2^-24 B
+// of the exact value; the scan's |q|^2 + |x|^2 - 2 q.x differs from the exact
+// value by at most (2d + 6) 2^-24 (|q|^2 + |x|^2), and |x|^2 <= 2 |q|^2 +
+// 2 |q - x|^2 <= 2 |q|^2 + 2 B (1 + (d + 2) 2^-23).  So
+//     B (1 + (d + 2) 2^-23) + 4 (d + 4) 2^-24 (3 |q|^2 + 3 B)
 // (rounded up; its square root, rounded up, for euclidean) bounds the k-th
 // smallest scan distance over the probes.  All ones when the first probe has
-// fewer than k live entries.
+// fewer than k live entries.  Eight lanes read a row together (10k queries x
+// 41 entries x 96: 352 us with a row per lane, whose loads touch 32 lines).
 __global__ void __launch_bounds__(128) k_pm_bound(SpfArgs a, const uint32_t *probe, const uint32_t *pcnt,
                                                   uint32_t nprobe, uint32_t k, uint32_t *qthr) {
-  extern __shared__ float bsm[];  // [4][cap] squared distances
+  extern __shared__ __align__(16) float bsm[];  // [4][cap] squared distances, [4][dpad] queries
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   float *sv = bsm + (size_t)warp * a.cap;
+  float *qs = bsm + (((size_t)4 * a.cap + 3) & ~(size_t)3) + (size_t)warp * a.dpad;
   for (uint32_t q = blockIdx.x * 4 + warp; q < a.nq; q += gridDim.x * 4) {
     uint32_t tb = 0xffffffffu;
     if (pcnt[q] > 0) {
       const uint32_t b = probe[(size_t)q * nprobe];
       const uint32_t n_e = min(a.len[b], a.cap);
       const float *qg = a.Q + (size_t)q * a.d;
-      float qq = 0.0f, xxm = 0.0f;
-      for (uint32_t i = lane; i < a.d; i += 32) qq = fmaf(__ldg(qg + i), __ldg(qg + i), qq);
+      float qq = 0.0f;
+      for (uint32_t i = lane; i < a.dpad; i += 32) {
+        const float x = i < a.d ? __ldg(qg + i) : 0.0f;
+        qs[i] = x;
+        qq = fmaf(x, x, qq);
+      }
+      __syncwarp();
       int live = 0;
       for (uint32_t e0 = 0; e0 < n_e; e0 += 32) {
-        const uint32_t e = e0 + lane;
-        const bool ok = e < n_e && !is_deleted(a.deleted, __ldg(a.ids + (size_t)b * a.cap + e));
-        float sd = 0.0f, xx = 0.0f;
-        if (ok) {
-          const float *x = reinterpret_cast<const float *>(a.codes + ((size_t)b * a.cap + e) * a.code_stride);
-#pragma unroll 8
-          for (uint32_t i = 0; i < a.d; ++i) {
-            const float xv = __ldg(x + i), t = __fsub_rn(__ldg(qg + i), xv);
-            sd = __fadd_rn(sd, __fmul_rn(t, t));
-            xx = fmaf(xv, xv, xx);
-          }
-        }
+        const uint32_t row = b * a.cap + min(e0 + lane, n_e - 1);
+        const bool ok = e0 + lane < n_e && !is_deleted(a.deleted, __ldg(a.ids + row));
+        const float sd = rows_distance<8, 0, MET_L2>(a.codes, a.code_stride, (a.code_stride / 16) / 8, qs, row,
+                                                     (int)min(32u, n_e - e0), lane, false, 0.0f);
         const uint32_t msk = __ballot_sync(kFull, ok);
         if (ok) sv[live + __popc(msk & lanemask_lt(lane))] = sd;
         live += __popc(msk);
-        xxm = fmaxf(xxm, xx);
       }
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        qq += __shfl_xor_sync(kFull, qq, o);
-        xxm = fmaxf(xxm, __shfl_xor_sync(kFull, xxm, o));
-      }
+      for (int o = 16; o > 0; o >>= 1) qq += __shfl_xor_sync(kFull, qq, o);
       __syncwarp();
       if (live >= (int)k) {
         uint32_t lo = 0, hi = 0xffffffffu;  // the k-th smallest: smallest v with #{ <= v} >= k
@@ -943,10 +939,10 @@ __global__ void __launch_bounds__(128) k_pm_bound(SpfArgs a, const uint32_t *pro
           if (c >= k) hi = mid;
           else lo = mid + 1;
         }
-        const float fd = (float)a.d;
+        const float fd = (float)a.d, B = ordered_float(lo);
         const float c1 = __fmul_ru(fd + 2.0f, 1.1920928955078125e-7f);  // (d + 2) 2^-23
-        const float c2 = __fmul_ru(4.0f * (fd + 4.0f), 5.9604644775390625e-8f);  // 4 (d + 4) 2^-24
-        float bound = __fadd_ru(__fmul_ru(ordered_float(lo), __fadd_ru(1.0f, c1)), __fmul_ru(c2, __fadd_ru(qq, xxm)));
+        const float c2 = __fmul_ru(12.0f * (fd + 4.0f), 5.9604644775390625e-8f);  // 3 * 4 (d + 4) 2^-24
+        float bound = __fadd_ru(__fmul_ru(B, __fadd_ru(1.0f, c1)), __fmul_ru(c2, __fadd_ru(qq, B)));
         if (a.metric == DG_L2) bound = __fsqrt_ru(bound);
         tb = ordered_bits(bound);
       }
@@ -957,163 +953,246 @@ __global__ void __launch_bounds__(128) k_pm_bound(SpfArgs a, const uint32_t *pro
   }
 }
 
+// Per query of a posting-major chunk (a warp each), what every item that holds
+// it needs: its FP16 row (dk halves, zero padded), |q|^2, the largest
+// coordinate (infinite when a coordinate is not exact in FP16).
+__global__ void __launch_bounds__(256) k_pm_queries(const float *__restrict__ Q, uint32_t nq, uint32_t d, uint32_t dk,
+                                                    __half *__restrict__ qh, float2 *__restrict__ qinfo) {
+  const int lane = threadIdx.x & 31;
+  const uint32_t nw = (gridDim.x * blockDim.x) >> 5;
+  for (uint32_t q = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; q < nq; q += nw) {
+    float s2 = 0.0f, mx = 0.0f;
+    for (uint32_t i = lane; i < dk; i += 32) {
+      const float x = i < d ? __ldg(Q + (size_t)q * d + i) : 0.0f;
+      bool ok;
+      qh[(size_t)q * dk + i] = __ushort_as_half(f16_exact(x, ok));
+      s2 = fmaf(x, x, s2);
+      mx = ok ? fmaxf(mx, fabsf(x)) : __int_as_float(0x7f800000);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      s2 += __shfl_xor_sync(kFull, s2, o);
+      mx = fmaxf(mx, __shfl_xor_sync(kFull, mx, o));
+    }
+    if (lane == 0) qinfo[q] = make_float2(s2, mx);
+  }
+}
+
+// One CTA (8 warps) per work item at a time: the item's queries (FP16 rows,
+// copied as they are) and a tile of the posting's entries in shared memory.
+// When the tile and the queries meet the exactness bounds above, the warps
+// split the 64 x 32 tile of dot products into 16 x 16 tensor-core blocks and
+// compare each distance with its query's bound in registers: about one in a
+// hundred passes and goes to the query's candidates in shared memory, so that
+// only those reach the k-best lists.  Other tiles take an FMA chain per pair:
+// warp w scores queries w, w + 8, ... against two entries per lane.  A CTA
+// that met such a tile stages f32 rows ahead for the next ones.
 // qthr[q] (ordered distance bits) is an upper bound of query q's final k-th
 // distance: k_pm_bound's, lowered to the k-th distance of any of its pair
 // lists that holds k keys.  Entries farther than it cannot reach the result, so
 // they are dropped before the pair-list insertion (keys at the bound stay,
 // ties included); the result does not depend on when bounds arrive.
-__global__ void __launch_bounds__(256) k_pm_scan_postings(SpfArgs a, const uint4 *items, const uint32_t *n_items,
-                                                          uint32_t *item_counter, const uint32_t *pair_q,
-                                                          uint64_t *pair_keys, uint32_t *pair_cnt, uint32_t k,
-                                                          uint32_t *qthr) {
+// Bound by the staging of the tiles (f32 rows in, FP16 out) and the barriers
+// around it: 300k x 96, 10k queries, 64 probes: 1762 us when every item
+// converted its queries and every distance went through shared memory to the
+// insertion.
+__global__ void __launch_bounds__(256, 3) k_pm_scan_postings(SpfArgs a, const uint4 *items, const uint32_t *n_items,
+                                                             uint32_t *item_counter, const uint32_t *pair_q,
+                                                             uint64_t *pair_keys, uint32_t *pair_cnt, uint32_t k,
+                                                             uint32_t *qthr, const __half *__restrict__ gqh,
+                                                             const float2 *__restrict__ gqinfo) {
   extern __shared__ __align__(16) uint8_t smem[];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   // query rows dpad floats; tile rows d + 4 floats: 16-byte rows whose float4
   // columns fall in distinct banks within each quarter warp
   const uint32_t dq = a.dpad, dt = a.d + 4, d4 = a.d / 4;
   const uint32_t ks = pm_ks(a.d), dk = ks - 8, kc = pm_kcap(k);
   float *qsm = reinterpret_cast<float *>(smem);                              // [kPmQ][dpad]
   float *tile = qsm + kPmQ * dq;                                             // [kPmT][d + 4]
-  uint32_t *tid = reinterpret_cast<uint32_t *>(tile + kPmT * dt);            // [kPmT] ids
-  float *xn = reinterpret_cast<float *>(tid + kPmT);                         // [kPmT] |x|^2
+  uint64_t *cand = reinterpret_cast<uint64_t *>(tile);                       // [kPmQ][kPmT] (tensor-core tiles)
+  uint32_t *tids = reinterpret_cast<uint32_t *>(tile + pm_tile_floats(a.d));  // [kPmT] ids
+  float *xn = reinterpret_cast<float *>(tids + kPmT);                        // [kPmT] |x|^2
   float *qn = xn + kPmT;                                                     // [kPmQ] |q|^2
-  uint64_t *lists = reinterpret_cast<uint64_t *>(qn + kPmQ);                 // [kPmQ][2][kc]
+  uint32_t *sq_id = reinterpret_cast<uint32_t *>(qn + kPmQ);                 // [kPmQ] queries
+  uint32_t *thr = sq_id + kPmQ;                                              // [kPmQ] bounds
+  uint32_t *ccnt = thr + kPmQ;                                               // [kPmQ] candidates
+  uint64_t *lists = reinterpret_cast<uint64_t *>(ccnt + kPmQ);               // [kPmQ][2][kc]
   uint64_t *cst = lists + (size_t)kPmQ * 2 * kc;                             // [8][32]
   uint16_t *qh = reinterpret_cast<uint16_t *>(cst + 8 * 32);                 // [kPmQ][ks] FP16 queries
   uint16_t *th = qh + kPmQ * ks;                                             // [kPmT][ks] FP16 tile
-  // [kPmQ][kPmT] tensor-core dot products, over the f32 tile once it is converted
-  float *dm = tile;
-  __shared__ uint32_t s_item, s_qbad, s_tbad, s_qmax, s_tmax;
+  __shared__ uint32_t s_item, s_tmax;
+  __shared__ float s_qmax;
   const uint32_t total = *n_items;
-  const bool sq = a.metric == DG_L2;
+  const bool root = a.metric == DG_L2;
   const uint32_t qh_s = (uint32_t)__cvta_generic_to_shared(qh), th_s = (uint32_t)__cvta_generic_to_shared(th);
+  bool ahead = false;  // the last tile was not exact: stage f32 rows at once
   while (true) {
-    if (threadIdx.x == 0) {
-      s_item = atomicAdd(item_counter, 1u);
-      s_qbad = 0u;
-      s_qmax = 0u;
-    }
+    if (tid == 0) s_item = atomicAdd(item_counter, 1u);
     __syncthreads();
     const uint32_t it = s_item;
-    __syncthreads();
     if (it >= total) break;
-    const uint4 item = items[it];
+    const uint4 item = __ldg(items + it);
     const uint32_t b = item.x, p0 = item.y, m = item.z;
-    {  // queries: f32 rows (zero padded to dpad) and FP16 rows (zero padded to dk, rows past m zero)
-      bool bad = false;
-      float mx = 0.0f;
-      for (uint32_t t = threadIdx.x; t < kPmQ * dk; t += blockDim.x) {
-        const uint32_t j = t / dk, i = t % dk;
-        const float x = (j < m && i < a.d) ? __ldg(a.Q + (size_t)pair_q[p0 + j] * a.d + i) : 0.0f;
-        bool ok;
-        qh[j * ks + i] = f16_exact(x, ok);
-        bad |= !ok;
-        mx = fmaxf(mx, fabsf(x));
-        if (j < m && i < dq) qsm[j * dq + i] = x;
-      }
-      for (uint32_t t = threadIdx.x; t < m * dq; t += blockDim.x)
-        if (t % dq >= dk) qsm[t] = 0.0f;  // dpad beyond the FP16 width
-      if (__syncthreads_or(bad) && threadIdx.x == 0) s_qbad = 1u;
-      if (mx > 0.0f) atomicMax(&s_qmax, __float_as_uint(mx));
+    // queries: FP16 rows (rows past m zero), norms, bounds
+    for (uint32_t t = tid; t < kPmQ * (dk / 8); t += 256) {
+      const uint32_t j = t / (dk / 8), i = t - j * (dk / 8);
+      const uint32_t q = j < m ? __ldg(pair_q + p0 + j) : 0u;
+      cp_async16(qh + j * ks + 8 * i, gqh + (size_t)q * dk + 8 * i, j < m ? 16u : 0u);
     }
-    __syncthreads();
-    // query norms: a warp per query, lanes over the coordinates
-    for (uint32_t j = warp; j < m; j += blockDim.x >> 5) {
-      float s2 = 0.0f;
-      for (uint32_t i = lane; i < a.d; i += 32) s2 = fmaf(qsm[j * dq + i], qsm[j * dq + i], s2);
+    cp_async_commit();
+    if (warp == 0) {
+      const uint32_t q = lane < (int)m ? __ldg(pair_q + p0 + lane) : 0u;
+      const float2 info = lane < (int)m ? __ldg(gqinfo + q) : make_float2(0.0f, 0.0f);
+      sq_id[lane] = q;
+      qn[lane] = info.x;
+      thr[lane] = lane < (int)m ? *reinterpret_cast<volatile uint32_t *>(qthr + q) : 0u;
+      ccnt[lane] = 0u;
+      float mx = info.y;
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) s2 += __shfl_xor_sync(kFull, s2, o);
-      if (lane == 0) qn[j] = s2;
+      for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(kFull, mx, o));
+      if (lane == 0) s_qmax = mx;
     }
+    cp_async_wait<0>();
+    bool have_q = false;  // f32 queries staged
+    auto stage_queries = [&]() {  // f32 rows, zero padded to dpad
+      for (uint32_t t = tid; t < m * dq; t += 256) {
+        const uint32_t j = t / dq, i = t - j * dq;
+        qsm[t] = i < a.d ? __ldg(a.Q + (size_t)pair_q[p0 + j] * a.d + i) : 0.0f;
+      }
+      have_q = true;
+    };
+    if (ahead) stage_queries();
     // this warp's queries: j = warp + 8 u (u < 4)
     int cur[4] = {0, 0, 0, 0}, size[4] = {0, 0, 0, 0};
     const uint32_t n_e = a.len[b];
     for (uint32_t e0 = 0; e0 < n_e; e0 += kPmT) {
       const uint32_t ne = min((uint32_t)kPmT, n_e - e0);
+      if (tid == 0) s_tmax = 0u;
       __syncthreads();  // the previous tile is consumed (and the queries are in place)
-      if (threadIdx.x == 0) {
-        s_tbad = 0u;
-        s_tmax = 0u;
-      }
-      {  // the tile: f32 rows and FP16 rows (rows past ne and columns past d are zero)
-        bool bad = false;
-        float mx = 0.0f;
-        const uint32_t k4 = dk / 4;
-        for (uint32_t t = threadIdx.x; t < kPmT * k4; t += blockDim.x) {
-          const uint32_t r = t / k4, c = t % k4;
-          float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-          if (r < ne && c < d4) {
-            v = __ldg(reinterpret_cast<const float4 *>(a.codes + (size_t)(b * a.cap + e0 + r) * a.code_stride) + c);
-            reinterpret_cast<float4 *>(tile + r * dt)[c] = v;
+      bool bad = false;
+      {  // the tile: four threads per row, six float4 of each in flight; FP16 rows (rows past ne, columns past d zero)
+        const uint32_t r = tid >> 2, c0 = tid & 3;
+        const float4 *x = reinterpret_cast<const float4 *>(a.codes + (size_t)(b * a.cap + e0 + r) * a.code_stride);
+        float mx = 0.0f, s2 = 0.0f;
+        for (uint32_t cb = c0; cb < dk / 4; cb += 24) {
+          float4 v[6];
+#pragma unroll
+          for (int i = 0; i < 6; ++i) {
+            const uint32_t c = cb + 4 * i;
+            v[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            if (r < ne && c < d4) v[i] = __ldg(x + c);
           }
-          bool o0, o1, o2, o3;
-          const uint32_t lo = f16_exact(v.x, o0) | ((uint32_t)f16_exact(v.y, o1) << 16);
-          const uint32_t hi = f16_exact(v.z, o2) | ((uint32_t)f16_exact(v.w, o3) << 16);
-          *reinterpret_cast<uint2 *>(th + r * ks + 4 * c) = make_uint2(lo, hi);
-          bad |= !(o0 && o1 && o2 && o3);
-          mx = fmaxf(mx, fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))));
+#pragma unroll
+          for (int i = 0; i < 6; ++i) {
+            const uint32_t c = cb + 4 * i;
+            if (c >= dk / 4) break;
+            if (ahead && r < ne && c < d4) reinterpret_cast<float4 *>(tile + r * dt)[c] = v[i];
+            bool o0, o1, o2, o3;
+            const uint32_t lo = f16_exact(v[i].x, o0) | ((uint32_t)f16_exact(v[i].y, o1) << 16);
+            const uint32_t hi = f16_exact(v[i].z, o2) | ((uint32_t)f16_exact(v[i].w, o3) << 16);
+            *reinterpret_cast<uint2 *>(th + r * ks + 4 * c) = make_uint2(lo, hi);
+            bad |= !(o0 && o1 && o2 && o3);
+            mx = fmaxf(mx, fmaxf(fmaxf(fabsf(v[i].x), fabsf(v[i].y)), fmaxf(fabsf(v[i].z), fabsf(v[i].w))));
+            s2 = fmaf(v[i].x, v[i].x, fmaf(v[i].y, v[i].y, fmaf(v[i].z, v[i].z, fmaf(v[i].w, v[i].w, s2))));
+          }
         }
-        for (uint32_t r = threadIdx.x; r < kPmT; r += blockDim.x) {
+        s2 += __shfl_xor_sync(kFull, s2, 1);
+        s2 += __shfl_xor_sync(kFull, s2, 2);
+        if (c0 == 0) {
+          xn[r] = s2;  // (exact where it is used: tensor-core tiles)
           uint32_t id = DG_PAD;
           if (r < ne) {
             id = __ldg(a.ids + b * a.cap + e0 + r);
             if (is_deleted(a.deleted, id)) id = DG_PAD;
           }
-          tid[r] = id;
+          tids[r] = id;
         }
-        if (__syncthreads_or(bad) && threadIdx.x == 0) s_tbad = 1u;
-        if (mx > 0.0f) atomicMax(&s_tmax, __float_as_uint(mx));
+        const uint32_t wm = __reduce_max_sync(kFull, __float_as_uint(mx));  // (mx >= 0: bits order as values)
+        if (lane == 0 && wm) atomicMax(&s_tmax, wm);
       }
-      __syncthreads();
-      // entry norms: four lanes per row (8 rows per warp pass), interleaved
-      // coordinates, so a quarter warp reads one row's consecutive words
-      for (uint32_t r0 = 8u * warp; r0 < ne; r0 += 8u * (blockDim.x >> 5)) {
-        const uint32_t r = r0 + (lane >> 2);
-        float s2 = 0.0f;
-        if (r < ne)
-          for (uint32_t i = lane & 3; i < a.d; i += 4) s2 = fmaf(tile[r * dt + i], tile[r * dt + i], s2);
-        s2 += __shfl_xor_sync(kFull, s2, 1);
-        s2 += __shfl_xor_sync(kFull, s2, 2);
-        if (r < ne && (lane & 3) == 0) xn[r] = s2;
-      }
-      const float qm = __uint_as_float(s_qmax), tm = __uint_as_float(s_tmax);
-      // (the dot products overwrite the f32 tile, which must hold kPmQ x kPmT floats)
-      const bool tc = !s_qbad && !s_tbad && dt >= (uint32_t)kPmQ && (float)a.d * qm * tm < kPmExactSum;
-      __syncthreads();  // xn read the f32 tile
-      float acc[4][2];
-#pragma unroll
-      for (int u = 0; u < 4; ++u) acc[u][0] = acc[u][1] = 0.0f;
+      const bool tbad = __syncthreads_or(bad);
+      // (an inexact query makes s_qmax infinite; the candidates overlay the f32 tile)
+      const bool tc = !tbad && (float)a.d * s_qmax * __uint_as_float(s_tmax) < kPmExactSum;
       if (tc) {
         // warp w: entries 16 (w % 4) .. +15 against queries 16 (w / 4) .. +15
         const uint32_t e16 = 16u * (warp & 3), q16 = 16u * (warp >> 2);
-        float c[2][4] = {{0.0f, 0.0f, 0.0f, 0.0f}, {0.0f, 0.0f, 0.0f, 0.0f}};
-        const uint32_t arow = e16 + (lane & 15), acol = (lane >> 4) * 8;
-        const uint32_t brow = q16 + (lane >> 4) * 8 + (lane & 7), bcol = ((lane >> 3) & 1) * 8;
-        for (uint32_t k0 = 0; k0 < dk; k0 += 16) {
-          uint32_t av[4], bv[4];
-          ldsm_x4(av, th_s + 2u * (arow * ks + k0 + acol));
-          ldsm_x4(bv, qh_s + 2u * (brow * ks + k0 + bcol));
-          mma_f16_16x8x16(c[0], av, bv[0], bv[1]);
-          mma_f16_16x8x16(c[1], av, bv[2], bv[3]);
-        }
-        // lane (g, t) holds entries g, g + 8 x queries 2t, 2t + 1 of each 8-query tile
-        const uint32_t g = lane >> 2, t2 = 2 * (lane & 3);
+        if (e16 < ne && q16 < m) {
+          float c[2][4] = {{0.0f, 0.0f, 0.0f, 0.0f}, {0.0f, 0.0f, 0.0f, 0.0f}};
+          const uint32_t arow = e16 + (lane & 15), acol = (lane >> 4) * 8;
+          const uint32_t brow = q16 + (lane >> 4) * 8 + (lane & 7), bcol = ((lane >> 3) & 1) * 8;
+          for (uint32_t k0 = 0; k0 < dk; k0 += 16) {
+            uint32_t av[4], bv[4];
+            ldsm_x4(av, th_s + 2u * (arow * ks + k0 + acol));
+            ldsm_x4(bv, qh_s + 2u * (brow * ks + k0 + bcol));
+            mma_f16_16x8x16(c[0], av, bv[0], bv[1]);
+            mma_f16_16x8x16(c[1], av, bv[2], bv[3]);
+          }
+          // lane (g, t) holds entries g, g + 8 x queries 2t, 2t + 1 of each 8-query tile
+          const uint32_t g = lane >> 2, t2 = 2 * (lane & 3);
+          const float xg[2] = {xn[e16 + g], xn[e16 + g + 8]};
+          const uint32_t ig[2] = {tids[e16 + g], tids[e16 + g + 8]};
 #pragma unroll
-        for (int nt = 0; nt < 2; ++nt) {
-          const uint32_t qc = q16 + 8 * nt + t2;
-          dm[qc * kPmT + e16 + g] = c[nt][0];
-          dm[(qc + 1) * kPmT + e16 + g] = c[nt][1];
-          dm[qc * kPmT + e16 + g + 8] = c[nt][2];
-          dm[(qc + 1) * kPmT + e16 + g + 8] = c[nt][3];
+          for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              const uint32_t qc = q16 + 8 * nt + t2 + (e & 1);
+              // |q - x|^2 = |q|^2 + |x|^2 - 2 q.x (exact on integer-valued data)
+              const float s0 = fmaxf(__fsub_rn(__fadd_rn(qn[qc], xg[e >> 1]), __fmul_rn(2.0f, c[nt][e])), 0.0f);
+              const float dv = root ? __fsqrt_rn(s0) : s0;
+              if (qc < m && ig[e >> 1] != DG_PAD && ordered_bits(dv) <= thr[qc])
+                cand[qc * kPmT + atomicAdd(ccnt + qc, 1u)] = make_key(dv, ig[e >> 1]);
+            }
         }
         __syncthreads();
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
           const uint32_t j = warp + 8 * u;
-          acc[u][0] = dm[j * kPmT + lane];
-          acc[u][1] = dm[j * kPmT + lane + 32];
+          if (j >= m) continue;  // warp-uniform
+          const int n = (int)ccnt[j];
+          if (n == 0) continue;
+          uint64_t *const bufs[2] = {lists + (size_t)j * 2 * kc, lists + (size_t)j * 2 * kc + kc};
+          for (int i0 = 0; i0 < n; i0 += 32)
+            insert_batch(i0 + lane < n ? cand[j * kPmT + i0 + lane] : kKeyInvalid, bufs, cur[u], size[u], (int)k,
+                         cst + warp * 32, lane);
+          __syncwarp();
+          if (lane == 0) {
+            ccnt[j] = 0u;
+            uint32_t tb = *reinterpret_cast<volatile uint32_t *>(qthr + sq_id[j]);
+            if (size[u] >= (int)k) {
+              const uint32_t nb = key_hi(bufs[cur[u]][k - 1]);
+              if (nb < tb) {
+                atomicMin(qthr + sq_id[j], nb);
+                tb = nb;
+              }
+            }
+            thr[j] = tb;
+          }
         }
       } else {
+        if (!ahead) {  // f32 rows of this tile
+          for (uint32_t t = tid; t < ne * d4; t += 256) {
+            const uint32_t r = t / d4, c = t - r * d4;
+            reinterpret_cast<float4 *>(tile + r * dt)[c] =
+                __ldg(reinterpret_cast<const float4 *>(a.codes + (size_t)(b * a.cap + e0 + r) * a.code_stride) + c);
+          }
+          ahead = true;
+        }
+        if (!have_q) stage_queries();
+        __syncthreads();
+        // entry norms: four lanes per row (8 rows per warp pass), interleaved
+        // coordinates, so a quarter warp reads one row's consecutive words
+        for (uint32_t r0 = 8u * warp; r0 < ne; r0 += 8u * 8u) {
+          const uint32_t r = r0 + (lane >> 2);
+          float s2 = 0.0f;
+          if (r < ne)
+            for (uint32_t i = lane & 3; i < a.d; i += 4) s2 = fmaf(tile[r * dt + i], tile[r * dt + i], s2);
+          s2 += __shfl_xor_sync(kFull, s2, 1);
+          s2 += __shfl_xor_sync(kFull, s2, 2);
+          if (r < ne && (lane & 3) == 0) xn[r] = s2;
+        }
+        float acc[4][2];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) acc[u][0] = acc[u][1] = 0.0f;
         const float4 *e0p = reinterpret_cast<const float4 *>(tile + (size_t)lane * dt);
         const float4 *e1p = reinterpret_cast<const float4 *>(tile + (size_t)(lane + 32) * dt);
 #pragma unroll 2
@@ -1129,26 +1208,28 @@ __global__ void __launch_bounds__(256) k_pm_scan_postings(SpfArgs a, const uint4
             }
           }
         }
-      }
-      const uint32_t id0 = tid[lane], id1 = tid[lane + 32];
+        __syncthreads();  // the norms are in place
+        const uint32_t id0 = tids[lane], id1 = tids[lane + 32];
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const uint32_t j = warp + 8 * u;
-        if (j >= m) continue;  // warp-uniform
-        uint64_t *const bufs[2] = {lists + (size_t)j * 2 * kc, lists + (size_t)j * 2 * kc + kc};
-        uint32_t *qt = qthr + pair_q[p0 + j];
-        const uint32_t tb = *reinterpret_cast<volatile uint32_t *>(qt);
-        // |q - x|^2 = |q|^2 + |x|^2 - 2 q.x (exact on integer-valued data)
-        const float qq = qn[j];
-        const float s0 = fmaxf(__fsub_rn(__fadd_rn(qq, xn[lane]), __fmul_rn(2.0f, acc[u][0])), 0.0f);
-        const float s1 = fmaxf(__fsub_rn(__fadd_rn(qq, xn[lane + 32]), __fmul_rn(2.0f, acc[u][1])), 0.0f);
-        const float d0 = sq ? __fsqrt_rn(s0) : s0, d1 = sq ? __fsqrt_rn(s1) : s1;
-        const bool k0 = id0 != DG_PAD && ordered_bits(d0) <= tb, k1 = id1 != DG_PAD && ordered_bits(d1) <= tb;
-        insert_batch(k0 ? make_key(d0, id0) : kKeyInvalid, bufs, cur[u], size[u], (int)k, cst + warp * 32, lane);
-        insert_batch(k1 ? make_key(d1, id1) : kKeyInvalid, bufs, cur[u], size[u], (int)k, cst + warp * 32, lane);
-        if (size[u] >= (int)k && lane == 0) {
-          const uint32_t nb = key_hi(bufs[cur[u]][k - 1]);
-          if (nb < tb) atomicMin(qt, nb);
+        for (int u = 0; u < 4; ++u) {
+          const uint32_t j = warp + 8 * u;
+          if (j >= m) continue;  // warp-uniform
+          uint64_t *const bufs[2] = {lists + (size_t)j * 2 * kc, lists + (size_t)j * 2 * kc + kc};
+          uint32_t *qt = qthr + sq_id[j];
+          const uint32_t tb = *reinterpret_cast<volatile uint32_t *>(qt);
+          const float qq = qn[j];
+          const float s0 = fmaxf(__fsub_rn(__fadd_rn(qq, xn[lane]), __fmul_rn(2.0f, acc[u][0])), 0.0f);
+          const float s1 = fmaxf(__fsub_rn(__fadd_rn(qq, xn[lane + 32]), __fmul_rn(2.0f, acc[u][1])), 0.0f);
+          const float d0 = root ? __fsqrt_rn(s0) : s0, d1 = root ? __fsqrt_rn(s1) : s1;
+          const bool k0 = id0 != DG_PAD && ordered_bits(d0) <= tb, k1 = id1 != DG_PAD && ordered_bits(d1) <= tb;
+          insert_batch(k0 ? make_key(d0, id0) : kKeyInvalid, bufs, cur[u], size[u], (int)k, cst + warp * 32, lane);
+          insert_batch(k1 ? make_key(d1, id1) : kKeyInvalid, bufs, cur[u], size[u], (int)k, cst + warp * 32, lane);
+          if (lane == 0) {
+            uint32_t nt = tb;
+            if (size[u] >= (int)k) nt = min(nt, key_hi(bufs[cur[u]][k - 1]));
+            if (nt < tb) atomicMin(qt, nt);
+            thr[j] = nt;
+          }
         }
       }
     }
@@ -1160,6 +1241,7 @@ __global__ void __launch_bounds__(256) k_pm_scan_postings(SpfArgs a, const uint4
       for (int i = lane; i < size[u]; i += 32) pair_keys[(size_t)(p0 + j) * k + i] = lst[i];
       if (lane == 0) pair_cnt[p0 + j] = (uint32_t)size[u];
     }
+    __syncthreads();  // the item's shared state is free
   }
 }
 
@@ -1653,8 +1735,11 @@ __global__ void __launch_bounds__(128) k_pm_merge(const uint32_t *probe_cnt, con
   }
 }
 
+// What the scan holds beyond the tile rows, queries and lists that decide
+// whether a search runs posting-major: bounds, counts, and small rows' candidates.
+static size_t pm_extra(uint32_t d) { return (size_t)3 * kPmQ * 4 + (pm_tile_floats(d) - (size_t)kPmT * (d + 4)) * 4; }
 static size_t pm_smem(uint32_t d, uint32_t dpad, uint32_t k) {
-  return ((size_t)kPmQ * dpad + (size_t)kPmT * (d + 4)) * 4 + (2 * kPmT + kPmQ) * 4 +
+  return ((size_t)kPmQ * dpad + pm_tile_floats(d)) * 4 + (2 * kPmT + 4 * kPmQ) * 4 +
          (size_t)kPmQ * 2 * pm_kcap(k) * 8 + 8 * 32 * 8 + (size_t)(kPmQ + kPmT) * pm_ks(d) * 2;
 }
 
@@ -1756,7 +1841,9 @@ static DgStatus pm_scan_chunk(DgSpfresh *s, const SpfArgs &ac, uint32_t nprobe, 
   if ((r = buf_reserve(s->pair_keys, npairs * k * 8)) != DG_OK) return r;
   if ((r = buf_reserve(s->pair_cnt, npairs * 4)) != DG_OK) return r;
   if ((r = buf_reserve(s->misc, 16)) != DG_OK) return r;
+  const uint32_t dk = pm_ks(s->d) - 8;
   if ((r = buf_reserve(s->qthr, (size_t)qn * 4)) != DG_OK) return r;
+  if ((r = buf_reserve(s->pm_q, (size_t)qn * (8 + dk * 2))) != DG_OK) return r;
   uint32_t *probe = (uint32_t *)s->probe.p, *pcnt = (uint32_t *)s->probe_cnt.p;
   uint32_t *pcount = (uint32_t *)s->pcount.p, *pstart = (uint32_t *)s->pstart.p, *pfill = (uint32_t *)s->pfill.p;
   uint32_t *istart = (uint32_t *)s->istart.p, *counter = (uint32_t *)s->misc.p;
@@ -1793,7 +1880,7 @@ static DgStatus pm_scan_chunk(DgSpfresh *s, const SpfArgs &ac, uint32_t nprobe, 
   DG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s->device));
   if (per_sm < 1) return fail(DG_ENOTSUP, "posting-major scan does not fit on an SM");
   uint32_t *qthr = (uint32_t *)s->qthr.p;
-  const size_t bsmem = (size_t)4 * s->cap * 4;
+  const size_t bsmem = (((size_t)4 * s->cap + 3) & ~(size_t)3) * 4 + (size_t)4 * s->dpad * 4;
   if (bsmem <= 160 * 1024) {
     DG_CUDA(cudaFuncSetAttribute(k_pm_bound, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bsmem));
     k_pm_bound<<<(unsigned)std::min<uint32_t>((qn + 3) / 4, 148 * 16), 128, bsmem, st>>>(ac, probe, pcnt, nprobe,
@@ -1801,9 +1888,13 @@ static DgStatus pm_scan_chunk(DgSpfresh *s, const SpfArgs &ac, uint32_t nprobe, 
   } else {
     DG_CUDA(cudaMemsetAsync(qthr, 0xff, (size_t)qn * 4, st));  // no bound: every entry goes to its pair list
   }
+  // FP16 rows first (16-byte aligned), then (|q|^2, largest coordinate)
+  __half *gqh = (__half *)s->pm_q.p;
+  float2 *gqinfo = (float2 *)((uint8_t *)s->pm_q.p + (size_t)qn * dk * 2);
+  k_pm_queries<<<(unsigned)std::min<uint32_t>((qn + 7) / 8, 148 * 16), 256, 0, st>>>(ac.Q, qn, s->d, dk, gqh, gqinfo);
   k_pm_scan_postings<<<per_sm * sms, 256, smem, st>>>(ac, (const uint4 *)s->items.p, istart + nb, counter,
                                                       (const uint32_t *)s->pair_q.p, (uint64_t *)s->pair_keys.p,
-                                                      (uint32_t *)s->pair_cnt.p, k, qthr);
+                                                      (uint32_t *)s->pair_cnt.p, k, qthr, gqh, gqinfo);
   k_pm_merge<<<(unsigned)std::min<uint32_t>((qn + 3) / 4, 148 * 16), 128, 0, st>>>(
       pcnt, (const uint32_t *)s->pos_of.p, qn, nprobe, (const uint64_t *)s->pair_keys.p,
       (const uint32_t *)s->pair_cnt.p, k, ac.out_ids, ac.out_d, ac.out_cnt);
@@ -1844,7 +1935,7 @@ DgStatus dg_spfresh_destroy(DgSpfresh *s) {
   for (void *p : s->allocs) cudaFree(p);
   for (DgIndex::Buf *b : {&s->q, &s->oids, &s->od, &s->ocnt, &s->route, &s->live_idx, &s->fr, &s->probe, &s->probe_cnt,
                           &s->pcount, &s->pstart, &s->pfill, &s->istart, &s->pair_q, &s->pos_of, &s->items,
-                          &s->pair_keys, &s->pair_cnt, &s->misc, &s->qthr})
+                          &s->pair_keys, &s->pair_cnt, &s->misc, &s->qthr, &s->pm_q})
     if (b->p) cudaFree(b->p);
   if (s->counter) cudaFree(s->counter);
   if (s->stream) cudaStreamDestroy(s->stream);
@@ -2170,7 +2261,7 @@ DgStatus dg_spfresh_search_batch(DgSpfresh *s, const DgSpfreshParams *p, const f
   const bool posting_major = s->nblocks >= 512 && s->quant == DG_Q_NONE &&
                              (s->metric == DG_L2 || s->metric == DG_L2SQ) && p->k <= (uint32_t)kPmK && nq >= 256 &&
                              (uint64_t)nq * nprobe >= 16ull * s->nblocks && s->nblocks < (1u << 22) && s->d % 4 == 0 &&
-                             pm_smem(s->d, s->dpad, p->k) <= 200 * 1024;
+                             pm_smem(s->d, s->dpad, p->k) <= 200 * 1024 + pm_extra(s->d);
   // DG_SPF_EXACT_ROUTE=1 routes with the exact FP32 kernel only (an A/B knob)
   static const bool exact_only = std::getenv("DG_SPF_EXACT_ROUTE") && atoi(std::getenv("DG_SPF_EXACT_ROUTE"));
   // batches of >= 256 queries under L2 with n_probe <= 64 and d <= 128 route on

@@ -1016,7 +1016,8 @@ __global__ void __launch_bounds__(256, 3) k_pm_scan_postings(SpfArgs a, const ui
   uint32_t *sq_id = reinterpret_cast<uint32_t *>(qn + kPmQ);                 // [kPmQ] queries
   uint32_t *thr = sq_id + kPmQ;                                              // [kPmQ] bounds
   uint32_t *ccnt = thr + kPmQ;                                               // [kPmQ] candidates
-  uint64_t *lists = reinterpret_cast<uint64_t *>(ccnt + kPmQ);               // [kPmQ][2][kc]
+  uint32_t *state = ccnt + kPmQ;                                             // [kPmQ] list size, low bit: buffer
+  uint64_t *lists = reinterpret_cast<uint64_t *>(state + kPmQ);              // [kPmQ][2][kc]
   uint64_t *cst = lists + (size_t)kPmQ * 2 * kc;                             // [8][32]
   uint16_t *qh = reinterpret_cast<uint16_t *>(cst + 8 * 32);                 // [kPmQ][ks] FP16 queries
   uint16_t *th = qh + kPmQ * ks;                                             // [kPmT][ks] FP16 tile
@@ -1046,7 +1047,7 @@ __global__ void __launch_bounds__(256, 3) k_pm_scan_postings(SpfArgs a, const ui
       sq_id[lane] = q;
       qn[lane] = info.x;
       thr[lane] = lane < (int)m ? *reinterpret_cast<volatile uint32_t *>(qthr + q) : 0u;
-      ccnt[lane] = 0u;
+      ccnt[lane] = state[lane] = 0u;
       float mx = info.y;
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(kFull, mx, o));
@@ -1062,8 +1063,6 @@ __global__ void __launch_bounds__(256, 3) k_pm_scan_postings(SpfArgs a, const ui
       have_q = true;
     };
     if (ahead) stage_queries();
-    // this warp's queries: j = warp + 8 u (u < 4)
-    int cur[4] = {0, 0, 0, 0}, size[4] = {0, 0, 0, 0};
     const uint32_t n_e = a.len[b];
     for (uint32_t e0 = 0; e0 < n_e; e0 += kPmT) {
       const uint32_t ne = min((uint32_t)kPmT, n_e - e0);
@@ -1143,31 +1142,6 @@ __global__ void __launch_bounds__(256, 3) k_pm_scan_postings(SpfArgs a, const ui
                 cand[qc * kPmT + atomicAdd(ccnt + qc, 1u)] = make_key(dv, ig[e >> 1]);
             }
         }
-        __syncthreads();
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const uint32_t j = warp + 8 * u;
-          if (j >= m) continue;  // warp-uniform
-          const int n = (int)ccnt[j];
-          if (n == 0) continue;
-          uint64_t *const bufs[2] = {lists + (size_t)j * 2 * kc, lists + (size_t)j * 2 * kc + kc};
-          for (int i0 = 0; i0 < n; i0 += 32)
-            insert_batch(i0 + lane < n ? cand[j * kPmT + i0 + lane] : kKeyInvalid, bufs, cur[u], size[u], (int)k,
-                         cst + warp * 32, lane);
-          __syncwarp();
-          if (lane == 0) {
-            ccnt[j] = 0u;
-            uint32_t tb = *reinterpret_cast<volatile uint32_t *>(qthr + sq_id[j]);
-            if (size[u] >= (int)k) {
-              const uint32_t nb = key_hi(bufs[cur[u]][k - 1]);
-              if (nb < tb) {
-                atomicMin(qthr + sq_id[j], nb);
-                tb = nb;
-              }
-            }
-            thr[j] = tb;
-          }
-        }
       } else {
         if (!ahead) {  // f32 rows of this tile
           for (uint32_t t = tid; t < ne * d4; t += 256) {
@@ -1208,38 +1182,58 @@ __global__ void __launch_bounds__(256, 3) k_pm_scan_postings(SpfArgs a, const ui
             }
           }
         }
-        __syncthreads();  // the norms are in place
+        __syncthreads();  // the norms are in place, the f32 tile is read
         const uint32_t id0 = tids[lane], id1 = tids[lane + 32];
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
           const uint32_t j = warp + 8 * u;
           if (j >= m) continue;  // warp-uniform
-          uint64_t *const bufs[2] = {lists + (size_t)j * 2 * kc, lists + (size_t)j * 2 * kc + kc};
-          uint32_t *qt = qthr + sq_id[j];
-          const uint32_t tb = *reinterpret_cast<volatile uint32_t *>(qt);
           const float qq = qn[j];
           const float s0 = fmaxf(__fsub_rn(__fadd_rn(qq, xn[lane]), __fmul_rn(2.0f, acc[u][0])), 0.0f);
           const float s1 = fmaxf(__fsub_rn(__fadd_rn(qq, xn[lane + 32]), __fmul_rn(2.0f, acc[u][1])), 0.0f);
           const float d0 = root ? __fsqrt_rn(s0) : s0, d1 = root ? __fsqrt_rn(s1) : s1;
-          const bool k0 = id0 != DG_PAD && ordered_bits(d0) <= tb, k1 = id1 != DG_PAD && ordered_bits(d1) <= tb;
-          insert_batch(k0 ? make_key(d0, id0) : kKeyInvalid, bufs, cur[u], size[u], (int)k, cst + warp * 32, lane);
-          insert_batch(k1 ? make_key(d1, id1) : kKeyInvalid, bufs, cur[u], size[u], (int)k, cst + warp * 32, lane);
-          if (lane == 0) {
-            uint32_t nt = tb;
-            if (size[u] >= (int)k) nt = min(nt, key_hi(bufs[cur[u]][k - 1]));
-            if (nt < tb) atomicMin(qt, nt);
-            thr[j] = nt;
+          if (id0 != DG_PAD && ordered_bits(d0) <= thr[j])
+            cand[j * kPmT + atomicAdd(ccnt + j, 1u)] = make_key(d0, id0);
+          if (id1 != DG_PAD && ordered_bits(d1) <= thr[j])
+            cand[j * kPmT + atomicAdd(ccnt + j, 1u)] = make_key(d1, id1);
+        }
+      }
+      __syncthreads();
+      // the candidates of queries warp, warp + 8, ... enter their lists (one copy
+      // of the insertion: four unrolled ones missed the instruction cache)
+#pragma unroll 1
+      for (uint32_t j = warp; j < m; j += 8) {
+        const int n = (int)ccnt[j];
+        if (n == 0) continue;
+        uint64_t *const bufs[2] = {lists + (size_t)j * 2 * kc, lists + (size_t)j * 2 * kc + kc};
+        int cur = (int)(state[j] & 1u), size = (int)(state[j] >> 1);
+#pragma unroll 1
+        for (int i0 = 0; i0 < n; i0 += 32)
+          insert_batch(i0 + lane < n ? cand[j * kPmT + i0 + lane] : kKeyInvalid, bufs, cur, size, (int)k,
+                       cst + warp * 32, lane);
+        __syncwarp();
+        if (lane == 0) {
+          ccnt[j] = 0u;
+          state[j] = ((uint32_t)size << 1) | (uint32_t)cur;
+          uint32_t tb = *reinterpret_cast<volatile uint32_t *>(qthr + sq_id[j]);
+          if (size >= (int)k) {
+            const uint32_t nb = key_hi(bufs[cur][k - 1]);
+            if (nb < tb) {
+              atomicMin(qthr + sq_id[j], nb);
+              tb = nb;
+            }
           }
+          thr[j] = tb;
         }
       }
     }
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const uint32_t j = warp + 8 * u;
-      if (j >= m) continue;
-      const uint64_t *lst = lists + (size_t)j * 2 * kc + (size_t)cur[u] * kc;
-      for (int i = lane; i < size[u]; i += 32) pair_keys[(size_t)(p0 + j) * k + i] = lst[i];
-      if (lane == 0) pair_cnt[p0 + j] = (uint32_t)size[u];
+    __syncwarp();
+#pragma unroll 1
+    for (uint32_t j = warp; j < m; j += 8) {
+      const int size = (int)(state[j] >> 1);
+      const uint64_t *lst = lists + ((size_t)j * 2 + (state[j] & 1u)) * kc;
+      for (int i = lane; i < size; i += 32) pair_keys[(size_t)(p0 + j) * k + i] = lst[i];
+      if (lane == 0) pair_cnt[p0 + j] = (uint32_t)size;
     }
     __syncthreads();  // the item's shared state is free
   }
@@ -1290,6 +1284,7 @@ __global__ void __launch_bounds__(1024) k_fr_mean(const float *__restrict__ C, c
   const uint32_t i = threadIdx.x & 127, rg = threadIdx.x >> 7;
   float acc = 0.0f;
   if (i < d)
+#pragma unroll 8
     for (uint32_t j = rg; j < m; j += 8) acc += __ldg(C + (size_t)__ldg(cidx + 1 + j) * dpad + i);
   part[rg][i] = acc;
   __syncthreads();
@@ -1413,7 +1408,7 @@ __global__ void __launch_bounds__(128) k_route_tcm(const __half *__restrict__ qh
                                                    const __half *__restrict__ ch, const __half *__restrict__ cl,
                                                    const float2 *__restrict__ cinfo,
                                                    const uint32_t *__restrict__ cidx, float *__restrict__ D,
-                                                   uint32_t ldd) {
+                                                   uint32_t ldd, float *__restrict__ G, uint32_t ldg) {
   constexpr int KD = 16 * KS, RS = KD + 8;  // staged row stride (halves): conflict-free ldmatrix
   constexpr int CH = KD / 8;                // 16-byte chunks per row
   extern __shared__ __align__(16) uint8_t smem[];
@@ -1493,20 +1488,35 @@ __global__ void __launch_bounds__(128) k_route_tcm(const __half *__restrict__ qh
     }
     // lane (g, t): queries qa, qb x centroids 2t, 2t + 1 of each 8-centroid n-tile
     const uint32_t j0 = (uint32_t)(t0 + tt) * kFrC;
+    const float inf = __int_as_float(0x7f800000);
+    float ga[8], gb[8];  // smallest value of each n-tile, rows qa and qb
 #pragma unroll
     for (int nt = 0; nt < 8; ++nt) {
       const int cc = 8 * nt + 2 * t;
       const uint32_t j = j0 + cc;
       const float2 c0 = tinfo[sb * kFrC + cc], c1 = tinfo[sb * kFrC + cc + 1];
+      const float2 va = make_float2(fmaf(ia.y * c0.y, acc[nt][0], __fadd_rn(ia.x, c0.x)),
+                                    fmaf(ia.y * c1.y, acc[nt][1], __fadd_rn(ia.x, c1.x)));
+      const float2 vb = make_float2(fmaf(ib.y * c0.y, acc[nt][2], __fadd_rn(ib.x, c0.x)),
+                                    fmaf(ib.y * c1.y, acc[nt][3], __fadd_rn(ib.x, c1.x)));
       if (j < nl) {  // j even, ldd a multiple of 4: the pair is 8-byte aligned (column j + 1 may be padding)
-        if (qa < nq)
-          *reinterpret_cast<float2 *>(D + (size_t)qa * ldd + j) =
-              make_float2(fmaf(ia.y * c0.y, acc[nt][0], __fadd_rn(ia.x, c0.x)),
-                          fmaf(ia.y * c1.y, acc[nt][1], __fadd_rn(ia.x, c1.x)));
-        if (qb < nq)
-          *reinterpret_cast<float2 *>(D + (size_t)qb * ldd + j) =
-              make_float2(fmaf(ib.y * c0.y, acc[nt][2], __fadd_rn(ib.x, c0.x)),
-                          fmaf(ib.y * c1.y, acc[nt][3], __fadd_rn(ib.x, c1.x)));
+        if (qa < nq) *reinterpret_cast<float2 *>(D + (size_t)qa * ldd + j) = va;
+        if (qb < nq) *reinterpret_cast<float2 *>(D + (size_t)qb * ldd + j) = vb;
+      }
+      ga[nt] = fminf(j < nl ? va.x : inf, j + 1 < nl ? va.y : inf);
+      gb[nt] = fminf(j < nl ? vb.x : inf, j + 1 < nl ? vb.y : inf);
+#pragma unroll
+      for (int o = 1; o <= 2; o <<= 1) {
+        ga[nt] = fminf(ga[nt], __shfl_xor_sync(kFull, ga[nt], o));
+        gb[nt] = fminf(gb[nt], __shfl_xor_sync(kFull, gb[nt], o));
+      }
+    }
+    if (t < 2) {  // lane t = 0 stores qa's eight minima, t = 1 qb's
+      const uint32_t q = t ? qb : qa;
+      if (q < nq) {
+        float4 *o = reinterpret_cast<float4 *>(G + (size_t)q * ldg + j0 / 8);
+        o[0] = t ? make_float4(gb[0], gb[1], gb[2], gb[3]) : make_float4(ga[0], ga[1], ga[2], ga[3]);
+        o[1] = t ? make_float4(gb[4], gb[5], gb[6], gb[7]) : make_float4(ga[4], ga[5], ga[6], ga[7]);
       }
     }
     __syncthreads();  // every warp is done with this stage before it is refilled
@@ -1520,13 +1530,14 @@ static size_t fr_tcm_smem(int ks) { return 2 * 2 * kFrC * (16 * (size_t)ks + 8) 
 // least the row's n-th smallest A), the live indices with A <= U + 2 E(q)
 // into a list, their exact distances, the n smallest (distance, slot) keys,
 // the probe_ratio cut of the query-major selection.
-__global__ void __launch_bounds__(128) k_fr_select(const float *__restrict__ D, uint32_t ldd, uint32_t nq,
+__global__ void __launch_bounds__(128) k_fr_select(const float *__restrict__ D, uint32_t ldd,
+                                                   const float *__restrict__ G, uint32_t ldg, uint32_t nq,
                                                    const float4 *__restrict__ qinfo, const float *__restrict__ Q,
                                                    uint32_t qstride, uint32_t d, const float *__restrict__ C,
                                                    uint32_t dpad, const uint32_t *__restrict__ cidx, int metric,
                                                    uint32_t nprobe, float probe_ratio, uint32_t *probe_out,
                                                    uint32_t *probe_cnt) {
-  __shared__ uint32_t lists[4][kFrCap];
+  __shared__ uint32_t lists[4][kFrCap], groups[4][kFrCap];
   __shared__ __align__(16) uint64_t keys[4][kFrCap];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t n = max(nprobe, 1u), nl = __ldg(cidx);
@@ -1536,8 +1547,14 @@ __global__ void __launch_bounds__(128) k_fr_select(const float *__restrict__ D, 
   const float inf = __int_as_float(0x7f800000);
   for (uint32_t q = blockIdx.x * 4 + warp; q < nq; q += gridDim.x * 4) {
     const float *row = D + (size_t)q * ldd;
-    const float4 *row4 = reinterpret_cast<const float4 *>(row);
-    const uint32_t n4 = nl / 4;
+    // the minima of eight centroids each stand in for the row while there are
+    // twice as many as probes: any n of them belong to n different centroids
+    const uint32_t ng = (nl + 7) / 8;
+    const bool by_group = ng >= 2 * n;
+    const float *seen = by_group ? G + (size_t)q * ldg : row;
+    const uint32_t ns = by_group ? ng : nl;
+    const float4 *seen4 = reinterpret_cast<const float4 *>(seen);
+    const uint32_t n4 = ns / 4;
     float bound = inf;
     if (nl > n) {
       // the four smallest values this lane sees
@@ -1554,7 +1571,7 @@ __global__ void __launch_bounds__(128) k_fr_select(const float *__restrict__ D, 
       for (; i + 96 < n4; i += 128) {  // four loads in flight per lane
         float4 v[4];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) v[u] = __ldg(row4 + i + 32 * u);
+        for (int u = 0; u < 4; ++u) v[u] = __ldg(seen4 + i + 32 * u);
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
           see(v[u].x);
@@ -1564,13 +1581,13 @@ __global__ void __launch_bounds__(128) k_fr_select(const float *__restrict__ D, 
         }
       }
       for (; i < n4; i += 32) {
-        const float4 v = __ldg(row4 + i);
+        const float4 v = __ldg(seen4 + i);
         see(v.x);
         see(v.y);
         see(v.z);
         see(v.w);
       }
-      if (4 * n4 + lane < nl) see(__ldg(row + 4 * n4 + lane));
+      if (4 * n4 + lane < ns) see(__ldg(seen + 4 * n4 + lane));
       // U: the n-th smallest of the 128 kept values (ordered bits, bisection)
       const uint32_t u0 = ordered_bits(t0), u1 = ordered_bits(t1), u2 = ordered_bits(t2), u3 = ordered_bits(t3);
       uint32_t lo = 0, hi = 0xffffffffu;
@@ -1582,32 +1599,63 @@ __global__ void __launch_bounds__(128) k_fr_select(const float *__restrict__ D, 
       }
       bound = __fadd_ru(ordered_float(lo), 2.0f * __ldg(qinfo + q).z);
     }
-    // the candidates: every live index with A <= bound (all of them when nl <= n)
-    int m = 0;
-    for (uint32_t i0 = 0; i0 < n4 + 1; i0 += 128) {  // four loads in flight per lane
-      float4 v[4];
+    // the entries of `seen` up to the bound (all of them when nl <= n): the
+    // candidates, or the groups that hold them
+    auto collect = [&](uint32_t *out) {
+      int cnt = 0;
+      for (uint32_t i0 = 0; i0 < n4 + 1; i0 += 128) {  // four loads in flight per lane
+        float4 v[4];
 #pragma unroll
-      for (int w = 0; w < 4; ++w) {
-        const uint32_t i = i0 + 32 * w + lane;
-        v[w] = make_float4(inf, inf, inf, inf);
-        if (i < n4) v[w] = __ldg(row4 + i);
-        else if (i == n4) {
-          if (4 * n4 < nl) v[w].x = __ldg(row + 4 * n4);
-          if (4 * n4 + 1 < nl) v[w].y = __ldg(row + 4 * n4 + 1);
-          if (4 * n4 + 2 < nl) v[w].z = __ldg(row + 4 * n4 + 2);
+        for (int w = 0; w < 4; ++w) {
+          const uint32_t i = i0 + 32 * w + lane;
+          v[w] = make_float4(inf, inf, inf, inf);
+          if (i < n4) v[w] = __ldg(seen4 + i);
+          else if (i == n4) {
+            if (4 * n4 < ns) v[w].x = __ldg(seen + 4 * n4);
+            if (4 * n4 + 1 < ns) v[w].y = __ldg(seen + 4 * n4 + 1);
+            if (4 * n4 + 2 < ns) v[w].z = __ldg(seen + 4 * n4 + 2);
+          }
+        }
+#pragma unroll
+        for (int w = 0; w < 4; ++w) {
+          const uint32_t i = i0 + 32 * w + lane;
+          const float vv[4] = {v[w].x, v[w].y, v[w].z, v[w].w};
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            const uint32_t j = 4 * i + u;
+            const bool keep = j < ns && (vv[u] <= bound || nl <= n);
+            const uint32_t km = __ballot_sync(kFull, keep);
+            const int pos = cnt + __popc(km & lanemask_lt(lane));
+            if (keep && pos < kFrCap) out[pos] = j;
+            cnt += __popc(km);
+          }
         }
       }
+      return cnt;
+    };
+    int m = 0;
+    if (!by_group) {
+      m = collect(lst);
+    } else {
+      uint32_t *glst = groups[warp];
+      const int gm = collect(glst);
+      __syncwarp();
+      m = gm > kFrCap ? kFrCap + 1 : 0;  // (too many for the list: the exact fallback below)
+      for (int x0 = 0; gm <= kFrCap && x0 < 8 * gm; x0 += 64) {  // eight lanes per group, two loads in flight
+        float v[2];
+        uint32_t j[2];
 #pragma unroll
-      for (int w = 0; w < 4; ++w) {
-        const uint32_t i = i0 + 32 * w + lane;
-        const float vv[4] = {v[w].x, v[w].y, v[w].z, v[w].w};
+        for (int w = 0; w < 2; ++w) {
+          const int x = x0 + 32 * w + lane;
+          j[w] = x < 8 * gm ? 8 * glst[x >> 3] + (x & 7) : nl;
+          v[w] = j[w] < nl ? __ldg(row + j[w]) : inf;
+        }
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const uint32_t j = 4 * i + u;
-          const bool keep = j < nl && (vv[u] <= bound || nl <= n);
+        for (int w = 0; w < 2; ++w) {
+          const bool keep = j[w] < nl && v[w] <= bound;
           const uint32_t km = __ballot_sync(kFull, keep);
           const int pos = m + __popc(km & lanemask_lt(lane));
-          if (keep && pos < kFrCap) lst[pos] = j;
+          if (keep && pos < kFrCap) lst[pos] = j[w];
           m += __popc(km);
         }
       }
@@ -1717,12 +1765,28 @@ __global__ void __launch_bounds__(128) k_pm_merge(const uint32_t *probe_cnt, con
   for (uint32_t q = blockIdx.x * 4 + warp; q < nq; q += gridDim.x * 4) {
     int cur = 0, size = 0;
     const uint32_t np = probe_cnt[q];
-    for (uint32_t i = 0; i < np; ++i) {
-      const uint32_t pos = pos_of[(size_t)q * nprobe + i];
-      const uint32_t c = pair_cnt[pos];
-      for (uint32_t j0 = 0; j0 < c; j0 += 32) {
-        const uint32_t j = j0 + lane;
-        insert_batch(j < c ? pair_keys[(size_t)pos * k + j] : kKeyInvalid, bufs, cur, size, (int)k, cst[warp], lane);
+    // 32 pairs at a time: their counts, then their keys packed 32 to a batch (most
+    // pairs keep a few keys or none; one pair at a time is a chain of three loads)
+    for (uint32_t i0 = 0; i0 < np; i0 += 32) {
+      const bool in = i0 + lane < np;
+      const uint32_t pos = in ? pos_of[(size_t)q * nprobe + i0 + lane] : 0u;
+      const uint32_t c = in ? pair_cnt[pos] : 0u;
+      uint32_t incl = c;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t t = __shfl_up_sync(kFull, incl, o);
+        if (lane >= o) incl += t;
+      }
+      const uint32_t total = __shfl_sync(kFull, incl, 31);
+      for (uint32_t t0 = 0; t0 < total; t0 += 32) {
+        const uint32_t t = t0 + lane;
+        uint32_t r = 0;  // the pair holding key t: pairs before it end at or before t
+#pragma unroll
+        for (int step = 16; step > 0; step >>= 1)
+          if (__shfl_sync(kFull, incl, r + step - 1) <= t) r += step;
+        const uint32_t first = __shfl_sync(kFull, incl - c, r), p = __shfl_sync(kFull, pos, r);
+        insert_batch(t < total ? pair_keys[(size_t)p * k + (t - first)] : kKeyInvalid, bufs, cur, size, (int)k,
+                     cst[warp], lane);
       }
     }
     const int count = min(size, (int)k);
@@ -1737,9 +1801,9 @@ __global__ void __launch_bounds__(128) k_pm_merge(const uint32_t *probe_cnt, con
 
 // What the scan holds beyond the tile rows, queries and lists that decide
 // whether a search runs posting-major: bounds, counts, and small rows' candidates.
-static size_t pm_extra(uint32_t d) { return (size_t)3 * kPmQ * 4 + (pm_tile_floats(d) - (size_t)kPmT * (d + 4)) * 4; }
+static size_t pm_extra(uint32_t d) { return (size_t)4 * kPmQ * 4 + (pm_tile_floats(d) - (size_t)kPmT * (d + 4)) * 4; }
 static size_t pm_smem(uint32_t d, uint32_t dpad, uint32_t k) {
-  return ((size_t)kPmQ * dpad + pm_tile_floats(d)) * 4 + (2 * kPmT + 4 * kPmQ) * 4 +
+  return ((size_t)kPmQ * dpad + pm_tile_floats(d)) * 4 + (2 * kPmT + 5 * kPmQ) * 4 +
          (size_t)kPmQ * 2 * pm_kcap(k) * 8 + 8 * 32 * 8 + (size_t)(kPmQ + kPmT) * pm_ks(d) * 2;
 }
 
@@ -1755,8 +1819,8 @@ struct FrPrep {
   float2 *cinfo;
   __half *ch, *cl, *qh, *ql;
   float4 *qinfo;
-  float *D;
-  uint32_t ldd;
+  float *D, *G;  // the A matrix, the smallest value of every eight columns
+  uint32_t ldd, ldg;
   int ks;  // 16-dimension steps of the padded rows (2, 4, 6 or 8)
 };
 
@@ -1766,8 +1830,10 @@ static DgStatus fr_prepare(DgSpfresh *s, const uint32_t *lidx, uint32_t chunk, c
   auto up = [](size_t x) { return (x + 255) & ~(size_t)255; };
   const size_t o_max = up(128 * 4), o_info = o_max + 256, o_h = o_info + up(nb * 8), o_l = o_h + up(nb * kd * 2),
                o_qi = o_l + up(nb * kd * 2), o_qh = o_qi + up((size_t)chunk * 16), o_ql = o_qh + up((size_t)chunk * kd * 2),
-               total = o_ql + up((size_t)chunk * kd * 2);
+               o_g = o_ql + up((size_t)chunk * kd * 2);
   fp->ldd = (uint32_t)((nb + 3) & ~(size_t)3);
+  fp->ldg = (uint32_t)((nb + 63) / 64 * 8);
+  const size_t total = o_g + (size_t)chunk * fp->ldg * 4;
   DgStatus r;
   if ((r = buf_reserve(s->fr, total)) != DG_OK) return r;
   if ((r = buf_reserve(s->route, (size_t)chunk * fp->ldd * 4)) != DG_OK) return r;
@@ -1781,6 +1847,7 @@ static DgStatus fr_prepare(DgSpfresh *s, const uint32_t *lidx, uint32_t chunk, c
   fp->qh = (__half *)(base + o_qh);
   fp->ql = (__half *)(base + o_ql);
   fp->D = (float *)s->route.p;
+  fp->G = (float *)(base + o_g);
   fp->ks = ks;
   k_fr_mean<<<1, 1024, 0, st>>>(s->centroids, lidx, s->d, s->dpad, fp->mu, fp->maxcc);
   k_fr_centroids<<<(unsigned)std::min<size_t>((nb + 7) / 8, 148 * 16), 256, 0, st>>>(
@@ -1796,7 +1863,7 @@ static DgStatus fr_matrix(const SpfArgs &ac, const FrPrep &fp, uint32_t nblocks,
   const uint32_t ntiles = (nblocks + kFrC - 1) / kFrC;
   dim3 grid((ac.nq + 63) / 64, std::max(1u, (ntiles + kFrTiles - 1) / kFrTiles));
   k_route_tcm<KS><<<grid, 128, smem, st>>>(fp.qh, fp.ql, fp.qinfo, ac.nq, fp.ch, fp.cl, fp.cinfo, ac.route_idx,
-                                           fp.D, fp.ldd);
+                                           fp.D, fp.ldd, fp.G, fp.ldg);
   DG_CUDA(cudaGetLastError());
   return DG_OK;
 }
@@ -1817,7 +1884,7 @@ static DgStatus fr_route(const SpfArgs &ac, const FrPrep &fp, uint32_t nprobe, u
   }
   if (r != DG_OK) return r;
   k_fr_select<<<(unsigned)std::min<uint32_t>((ac.nq + 3) / 4, 148 * 16), 128, 0, st>>>(
-      fp.D, fp.ldd, ac.nq, fp.qinfo, ac.Q, ac.d, ac.d, ac.centroids, ac.dpad, ac.route_idx, ac.metric, nprobe,
+      fp.D, fp.ldd, fp.G, fp.ldg, ac.nq, fp.qinfo, ac.Q, ac.d, ac.d, ac.centroids, ac.dpad, ac.route_idx, ac.metric, nprobe,
       ac.probe_ratio, probe, pcnt);
   DG_CUDA(cudaGetLastError());
   return DG_OK;

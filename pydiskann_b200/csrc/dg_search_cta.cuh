@@ -75,7 +75,7 @@ __device__ __forceinline__ int cta_sync_count(bool v) {
   return NW == 1 ? __popc(__ballot_sync(kFull, v)) : __syncthreads_count(v);
 }
 
-// Candidates a warp takes at a time.  16 keep a quarter (an eighth, a half) of
+// Candidates a warp takes at a time.  8 long rows of an eighth, or 16, keep a quarter (an eighth, a half) of
 // an expansion in flight at once.  32 where a lane scores a whole code, and
 // for a warp that has the expansion to itself, unless its rows are long (8
 // lanes per row): two tiles of 16 short rows wait for memory once, not twice
@@ -85,6 +85,7 @@ template <int NW, int TRAV, int LPR, bool TC>
 constexpr int cta_batch() {
   if (TRAV == TRAV_PQ || TRAV == TRAV_RABITQ) return 32;
   const bool rows = TRAV == TRAV_F32 || TRAV == TRAV_F16 || (TRAV == TRAV_BF16 && !TC);
+  if (NW == 8 && rows && LPR == 8) return 8;
   return NW == 1 && !(rows && LPR == 8) ? 32 : 16;
 }
 
@@ -97,14 +98,14 @@ __device__ __forceinline__ float cta_distance(const SearchArgs &a, uint8_t *sm, 
   if constexpr (B == 32) {
     return batch_distance<TRAV, MET, LPR, TC>(a, sm, Ly, cand, cnt, lane, qq);
   } else if constexpr (TRAV == TRAV_F32) {
-    return rows_distance16<LPR, 0, MET>(reinterpret_cast<const uint8_t *>(a.vec_f32), a.dpad * 4, (a.dpad / 4) / LPR,
+    return rows_distance_few<B == 8 ? 2 : LPR / 2, LPR, 0, MET>(reinterpret_cast<const uint8_t *>(a.vec_f32), a.dpad * 4, (a.dpad / 4) / LPR,
                                         qs, cand, cnt, lane, sq, qq);
   } else if constexpr (TRAV == TRAV_BF16 && !TC) {
-    return rows_distance16<LPR, 1, MET>(reinterpret_cast<const uint8_t *>(a.vec_bf16), a.dpad * 2,
+    return rows_distance_few<B == 8 ? 2 : LPR / 2, LPR, 1, MET>(reinterpret_cast<const uint8_t *>(a.vec_bf16), a.dpad * 2,
                                         (a.dpad / 8) / LPR, qs, cand, cnt, lane, sq, qq);
   } else if constexpr (TRAV == TRAV_F16) {
     const float *qx = MET == MET_L2 ? reinterpret_cast<const float *>(sm + Ly.prov) : qs;
-    return rows_distance16<LPR, 2, MET>(a.codes, a.code_stride, (a.code_stride / 16) / LPR, qx, cand, cnt, lane, sq,
+    return rows_distance_few<B == 8 ? 2 : LPR / 2, LPR, 2, MET>(a.codes, a.code_stride, (a.code_stride / 16) / LPR, qx, cand, cnt, lane, sq,
                                         qq);
   } else {
     return batch_distance<TRAV, MET, LPR, TC, true>(a, sm, Ly, cand, cnt, lane, qq);
@@ -363,8 +364,6 @@ __device__ inline void search_cta(const SearchArgs &a, uint32_t q, uint8_t *sm, 
   if (!FILT) lists[1].size = 0;
   int next = 0;                    // every list entry below it is expanded (warp 0)
   uint32_t n_exp = 0, n_dist = 0;  // warp 0's
-  const bool adj_pf = a.R % 4 == 0;  // rows of whole 16-byte blocks
-  const uint32_t adj_bytes = a.R * 4;
   if (tid == 0) {
     stage[0] = a.medoid;
     vt.test_and_set(a.medoid);
@@ -400,8 +399,6 @@ __device__ inline void search_cta(const SearchArgs &a, uint32_t q, uint8_t *sm, 
       if (TRAV != TRAV_F32 && a.code_limit < a.n && lane < cnt && cand >= a.code_limit)
         d = exact_row_distance<MET>(a, qs, cand, qq);
       const uint64_t key = lane < cnt ? make_key(d, cand) : kKeyInvalid;
-      // most keys that enter the list are expanded later: their neighbour lists go to L2
-      if (adj_pf && key < thr) prefetch_row(reinterpret_cast<const uint8_t *>(a.adj + (size_t)cand * a.R), 0, adj_bytes);
       cta_survive<NW>(lists[0], key, key < thr, ctl + CTL_CNT, lane);
       if (FILT && filtered)
         cta_survive<NW>(lists[1], key, lane < cnt && key < rthr && allow(cand, lab), ctl + CTL_CNTR, lane);
@@ -464,7 +461,7 @@ __device__ inline void search_cta(const SearchArgs &a, uint32_t q, uint8_t *sm, 
     for (int g0 = 16 * warp; g0 < nr; g0 += 16 * NW) {
       const int cnt = min(16, nr - g0);
       const uint32_t cand = lane < cnt ? key_id(src[g0 + lane]) : 0u;
-      const float d = rows_distance16<8, 0, MET>(reinterpret_cast<const uint8_t *>(a.vec_f32), a.dpad * 4,
+      const float d = rows_distance_few<4, 8, 0, MET>(reinterpret_cast<const uint8_t *>(a.vec_f32), a.dpad * 4,
                                                  (a.dpad / 4) / 8, qs, cand, cnt, lane, a.metric == DG_L2, qq);
       if (lane < cnt) tmp[g0 + lane] = make_key_payload(d, (uint32_t)(g0 + lane));
     }

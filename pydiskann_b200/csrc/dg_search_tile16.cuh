@@ -7,7 +7,7 @@
 namespace dg {
 
 // 16-byte loads in flight per lane: kTileLoads, spread over the row slots of
-// rows_distance16 or over the two rows of a tensor-core tile (4 KB per warp).
+// rows_distance_few or over the two rows of a tensor-core tile (4 KB per warp).
 // The rest of longer rows is asked for in L2 at the same time, so that only a
 // row's first round waits for DRAM.
 constexpr int kTileLoads = 8;
@@ -17,15 +17,15 @@ __device__ __forceinline__ void prefetch_row(const uint8_t *row, uint32_t from, 
   asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(row + from), "r"(to - from));
 }
 
-// rows_distance for at most 16 candidates: LPR / 2 row slots instead of LPR,
-// several 16-byte rounds of each in flight.  Every row is summed in the order of
+// rows_distance for at most S * 32 / LPR candidates: S row slots instead of
+// LPR, kTileLoads / S 16-byte rounds of each in flight.  Every row is summed in the order of
 // rows_distance (per lane over its chunks, then over lanes 4, 2, 1 apart), so
 // the distances are the same bits.
-template <int LPR, int ELEM, int MET>
-__device__ __forceinline__ float rows_distance16(const uint8_t *__restrict__ rows, uint32_t stride, int loads,
+template <int S, int LPR, int ELEM, int MET>
+__device__ __forceinline__ float rows_distance_few(const uint8_t *__restrict__ rows, uint32_t stride, int loads,
                                                  const float *qs, uint32_t cand, int cnt, int lane, bool sqrt_l2,
                                                  float qq) {
-  constexpr int RPI = 32 / LPR, S = LPR / 2;
+  constexpr int RPI = 32 / LPR;
   constexpr int EPC = Chunk<ELEM>::EPC;
   constexpr int U = kTileLoads / S;  // rounds in flight
   const int g = lane / LPR, r = lane % LPR;
@@ -79,10 +79,12 @@ __device__ __forceinline__ float rows_distance16(const uint8_t *__restrict__ row
       }
     }
   }
-  // lanes 4 (2, 1) apart first, then the transposed reduction over the S slots
+  // lanes LPR / 2 .. S apart first, then the transposed reduction over the S slots
   auto reduce = [&](float (&p)[S]) {
 #pragma unroll
-    for (int i = 0; i < S; ++i) p[i] += __shfl_xor_sync(kFull, p[i], S);
+    for (int o = LPR / 2; o >= S; o >>= 1)
+#pragma unroll
+      for (int i = 0; i < S; ++i) p[i] += __shfl_xor_sync(kFull, p[i], o);
     return transpose_reduce<S>(p, lane);
   };
   float a = reduce(sa), b = 0.0f;

@@ -1118,8 +1118,6 @@ DgStatus dg_pq_train(const float *X, uint64_t n, uint32_t dim, uint32_t M, uint3
     for (uint64_t i = 0; i < n; ++i) rows[i] = i;
   }
   const uint32_t ns = (uint32_t)rows.size();
-  std::vector<float> hs((size_t)ns * dim);
-  for (uint32_t i = 0; i < ns; ++i) std::copy(X + rows[i] * dim, X + rows[i] * dim + dim, hs.begin() + (size_t)i * dim);
   cudaStream_t st;
   DG_CUDA(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
   float *S = nullptr, *cb = nullptr, *mind = nullptr;
@@ -1129,7 +1127,7 @@ DgStatus dg_pq_train(const float *X, uint64_t n, uint32_t dim, uint32_t M, uint3
   DgStatus s = DG_OK;
   const size_t cbn = (size_t)M * K * ds;
   const uint32_t nblk = (ns + kSeedPts - 1) / kSeedPts;
-  if (cudaMallocAsync(&S, hs.size() * 4, st) != cudaSuccess || cudaMallocAsync(&cb, cbn * 4, st) != cudaSuccess ||
+  if (cudaMallocAsync(&S, (size_t)ns * dim * 4, st) != cudaSuccess || cudaMallocAsync(&cb, cbn * 4, st) != cudaSuccess ||
       cudaMallocAsync(&mind, (size_t)M * ns * 4, st) != cudaSuccess ||
       cudaMallocAsync(&sums, cbn * 8, st) != cudaSuccess ||
       cudaMallocAsync(&counts, (size_t)M * K * 4, st) != cudaSuccess ||
@@ -1137,16 +1135,16 @@ DgStatus dg_pq_train(const float *X, uint64_t n, uint32_t dim, uint32_t M, uint3
       cudaMallocAsync(&done, (size_t)M * 4, st) != cudaSuccess ||
       cudaMallocAsync(&codes, (size_t)M * ns, st) != cudaSuccess)
     s = fail(DG_ENOMEM, "pq training staging");
+  if (s == DG_OK) s = upload_rows_f32(X, ns, dim, dim, S, st, rows.data());
   if (s == DG_OK) {
-    cudaMemcpyAsync(S, hs.data(), hs.size() * 4, cudaMemcpyHostToDevice, st);
     // k-means++ seeding (src/pq.rs:301-341)
     cudaMemsetAsync(done, 0, (size_t)M * 4, st);
     const uint32_t keff = std::min<uint32_t>(K, ns);
     std::vector<float> hcb(cbn);
     for (uint32_t m = 0; m < M; ++m) {
       const uint32_t first = (uint32_t)(((unsigned __int128)rand4(seed, 0x6b6c, m, 0) * ns) >> 64);
-      std::copy(hs.begin() + (size_t)first * dim + m * ds, hs.begin() + (size_t)first * dim + m * ds + ds,
-                hcb.begin() + (size_t)m * K * ds);
+      const float *x = X + rows[first] * dim + m * ds;
+      std::copy(x, x + ds, hcb.begin() + (size_t)m * K * ds);
     }
     cudaMemcpyAsync(cb, hcb.data(), cbn * 4, cudaMemcpyHostToDevice, st);
     for (uint32_t c = 1; c < keff; ++c)

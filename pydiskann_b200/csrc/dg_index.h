@@ -102,7 +102,7 @@ DgStatus order_queries(const DgIndex *idx, const float *Q, uint32_t nq, uint32_t
 DgStatus to_device(DgIndex *idx, void **dst, const void *src, size_t bytes);
 // Rows of d floats from the host into [n][dpad] device rows, zero padded.
 DgStatus upload_rows_f32(const float *host, uint64_t n, uint32_t d, uint32_t dpad, float *dev,
-                         cudaStream_t st);
+                         cudaStream_t st, const uint64_t *rows = nullptr);
 // Kernels used by the attach/encode entry points (dg_build.cu).
 DgStatus encode_pq_device(const float *vec, uint64_t n, uint32_t d, uint32_t dpad, uint32_t M,
                           uint32_t K, const float *cb, uint8_t *codes, uint32_t stride,

@@ -62,3 +62,25 @@ def test_vamana_prune_batches(oracle, d, centres, sigma, R, Lb, shift):
     adj, med = dg.build_graph(X, R, Lb, 1.2, seed=5)
     want, _ = oracle.build_vamana(X, R, Lb, 1.2, seed=5, medoid_id=med)
     assert np.array_equal(adj, want)
+
+
+@pytest.mark.parametrize("n,d", [(11_000, 100), (40_000, 33), (9_000, 128)])
+def test_staged_upload(n, d):
+    """Uploads of several pinned pieces, rows padded on the device or not, from two threads at
+    once (one of them takes the plain copy): the rows come back as their own nearest neighbours."""
+    import threading
+
+    X = np.random.default_rng(n).permutation(n * d).reshape(n, d).astype(np.float32)
+    pick = np.linspace(0, n - 1, 50).astype(int)
+    out = [None, None]
+
+    def work(i):
+        out[i] = dg.exact_knn(X, X[pick], 1)
+
+    ts = [threading.Thread(target=work, args=(i,)) for i in range(2)]
+    for t in ts:
+        t.start()
+    for t in ts:
+        t.join()
+    for ids, ds in out:
+        assert np.array_equal(ids[:, 0], pick) and not ds.any()

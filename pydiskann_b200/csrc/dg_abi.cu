@@ -466,21 +466,24 @@ static DgIndex::Schedule schedule_of(DgIndex *idx, int trav, int lcap, bool filt
     std::lock_guard<std::mutex> lk(idx->mu);
     if (idx->forcing) {
       sc = idx->force;
+      sc.chosen = true;
       idx->last_key = tune_key(trav, lcap, filt);
     } else {
       auto it = idx->tuned.find(tune_key(trav, lcap, filt));
-      if (it != idx->tuned.end()) sc = it->second;
+      if (it != idx->tuned.end()) {
+        sc = it->second;
+        sc.chosen = true;
+      }
     }
   }
-  if (const char *e = std::getenv("DG_HBITS")) sc.hbits = (uint32_t)std::max(6, std::min(14, atoi(e)));
+  if (const char *e = std::getenv("DG_HBITS")) {
+    sc.hbits = (uint32_t)std::max(6, std::min(14, atoi(e)));
+    sc.chosen = true;
+  }
   if (const char *e = std::getenv("DG_ORDER")) sc.order = atoi(e) != 0;
   if (const char *e = std::getenv("DG_OCC_PCT")) sc.occ_pct = (uint32_t)std::max(1, std::min(100, atoi(e)));
   if (const char *e = std::getenv("DG_WPB")) sc.wpb = atoi(e) == 1 ? 1u : atoi(e) == 2 ? 2u : 4u;
   return sc;
-}
-
-static uint32_t visited_bits(DgIndex *idx, int trav, int lcap, bool filt, uint32_t maxL) {
-  return schedule_of(idx, trav, lcap, filt, maxL).hbits;
 }
 
 static void index_state(const DgIndex *idx, SearchArgs &a) {
@@ -523,28 +526,40 @@ static uint32_t traversal_row_bytes(const DgIndex *idx, int trav) {
 // short (int8 128-d, beam 40: 231 against 247 us for 16 queries, 344 against
 // 472 for 740; FP32 128-d: 369 against 255 for 16, 817 against 637 for 1200,
 // 833 against 822 for 2000; 768-d int8: 912 against 327 for 16).
+//
+// A large batch whose states leave room for fewer than 12 queries per SM takes
+// half the default visited table: a forgotten id only costs its distance
+// again (5000 PQ queries, beam 128, 2^11 -> 2^10 words: 3215 -> 2630 us; 4000
+// 768-d int8 cosine queries, beams up to 256, 2^12 -> 2^11: 7926 -> 6757 us;
+// one step more: 2618 and 7770).
 struct SearchPlan {
   WarpLayout Ly;
+  uint32_t hbits, hB;   // visited table: log2 words, id bits
   uint32_t cta;         // warps of the CTA a query takes, 0 = register-list kernel
   bool tc;              // BF16 rows take tensor-core distances
   uint32_t limit_smem;  // what decides whether the search is accepted, whichever kernel runs
 };
 static SearchPlan plan_search(const DgIndex *idx, int trav, int lcap, bool filt, uint64_t need, uint32_t search_k,
-                              bool reranked, uint32_t hbits, uint32_t wpb, uint32_t nq) {
+                              bool reranked, const DgIndex::Schedule &sc, uint32_t nq) {
   SearchPlan P;
+  P.hbits = sc.hbits;
   const bool decode = (trav == TRAV_RABITQ || trav == TRAV_INT8) && met_kind(idx->metric) != MET_L2;
-  const WarpLayout reg = warp_layout(trav, lcap, filt, hbits, idx->dpad, idx->pq_M, idx->pq_K, idx->rq_padded, decode,
-                                     idx->R, true);
-  P.limit_smem = reg.total * ((wpb == 1 || wpb == 2) ? wpb : 4u);
+  const WarpLayout reg = warp_layout(trav, lcap, filt, sc.hbits, idx->dpad, idx->pq_M, idx->pq_K, idx->rq_padded,
+                                     decode, idx->R, true);
+  P.limit_smem = reg.total * ((sc.wpb == 1 || sc.wpb == 2) ? sc.wpb : 4u);
   P.tc = lcap == 64 && !filt;
   // a label-free query of a filtered batch on an index with tombstones may hold
   // more than the labelled ones (tombstone_config)
   const uint64_t tneed = idx->tomb && idx->ntomb > 0 ? search_k + std::min<uint64_t>(idx->ntomb, need) : 0;
   const uint32_t rcap = filt ? search_k : 0, wcap = (uint32_t)std::min<uint64_t>(std::max(need, tneed), 1024);
-  P.Ly = cta_layout(trav, wcap, rcap, reranked ? std::min(search_k, filt ? rcap : wcap) : 0, filt, hbits, idx->dpad,
-                    idx->pq_M, idx->pq_K, idx->rq_padded, decode, idx->R);
   const uint32_t row = traversal_row_bytes(idx, trav), sms = (uint32_t)idx->sms;
-  const uint32_t room = 227u * 1024u / (P.Ly.total + 1024u);  // queries whose state an SM holds
+  auto fit = [&](uint32_t hbits) {  // the layout, and the queries whose state an SM holds
+    P.Ly = cta_layout(trav, wcap, rcap, reranked ? std::min(search_k, filt ? rcap : wcap) : 0, filt, hbits, idx->dpad,
+                      idx->pq_M, idx->pq_K, idx->rq_padded, decode, idx->R);
+    return 227u * 1024u / (P.Ly.total + 1024u);
+  };
+  uint32_t room = fit(P.hbits);
+  if (!sc.chosen && nq > 5 * sms && room < 12 && P.hbits > 10) room = fit(--P.hbits);
   // traversals whose lone warp takes 32 candidates at a time (cta_batch)
   const bool short_rows = trav == TRAV_INT8 || trav == TRAV_FP8 || trav == TRAV_PQ || trav == TRAV_RABITQ ||
                           ((trav == TRAV_BF16 || trav == TRAV_F16) && lanes_per_row(idx->dpad / 8) != 8);
@@ -556,7 +571,13 @@ static SearchPlan plan_search(const DgIndex *idx, int trav, int lcap, bool filt,
     const bool long_rows = row >= 256 || idx->dpad >= 512;
     if (!long_rows || nq > (row >= 512 || idx->dpad >= 512 ? 8 : 5) * sms || room == 0) P.cta = 0;
   }
-  if (P.cta == 0) P.Ly = reg;
+  if (P.cta == 0) {
+    P.Ly = reg;
+    P.hbits = sc.hbits;
+  }
+  P.hB = 1;
+  while (P.hB < 32 && (1ull << P.hB) < idx->n) ++P.hB;
+  P.hB = std::max(P.hB, P.hbits);
   return P;
 }
 
@@ -698,10 +719,6 @@ DgStatus dg_search_batch(DgIndex *idx, const DgSearchParams *p, const float *que
   // and CTAs per SM, as dg_index_autotune measured fastest for this kind of
   // search (defaults otherwise); DG_HBITS overrides the table size
   const DgIndex::Schedule sched = schedule_of(idx, trav, lcap, filt, maxL);
-  const uint32_t hbits = sched.hbits;
-  uint32_t hB = 1;
-  while (hB < 32 && (1ull << hB) < idx->n) ++hB;
-  hB = std::max(hB, hbits);
 
   std::lock_guard<std::mutex> lk(idx->mu);
   DG_CUDA(cudaSetDevice(idx->device));
@@ -744,8 +761,6 @@ DgStatus dg_search_batch(DgIndex *idx, const DgSearchParams *p, const float *que
   a.k = p->k;
   a.L = p->beam_width;
   a.rerank = p->rerank_size;
-  a.hbits = hbits;
-  a.hB = hB;
   if (any_filter) {
     if ((s = stage_copy(sl.fops, p->filter_ops, (size_t)total_ops * sizeof(DgFilterOp), st)) != DG_OK) return s;
     a.fops = (const DgFilterOp *)sl.fops.p;
@@ -826,8 +841,10 @@ DgStatus dg_search_batch(DgIndex *idx, const DgSearchParams *p, const float *que
       aa.perm = perm + q0;
     }
     DG_CUDA(cudaMemsetAsync(aa.counter, 0, 4, ss));
-    const SearchPlan P = plan_search(idx, trav, lcap, filt, need, search_k, reranked, hbits, sched.wpb, nq);
+    const SearchPlan P = plan_search(idx, trav, lcap, filt, need, search_k, reranked, sched, nq);
     aa.limit_smem = P.limit_smem;
+    aa.hbits = P.hbits;
+    aa.hB = P.hB;
     switch (trav) {
       case TRAV_F32: return launch_search_f32(aa, P.Ly, met, lpr, P.cta, P.tc, filt, ss, &info);
       case TRAV_BF16: return launch_search_bf16(aa, P.Ly, met, lpr, P.cta, P.tc, filt, ss, &info);
@@ -1161,10 +1178,8 @@ extern "C" DgStatus dg_search_batch_static(DgIndex *idx, const DgSearchParams *p
   const int lcap = need <= 64 ? 64 : need <= 256 ? 256 : need <= 1024 ? 1024 : 0;
   if (!lcap) return fail(DG_ENOTSUP, "beam width / expanded beam above 1024 is not supported");
   if (reranked && !filt && search_k > 1024) return fail(DG_ENOTSUP, "rerank size above 1024");
-  const uint32_t hbits = visited_bits(idx, trav, lcap, filt, maxL);
-  uint32_t hB = 1;
-  while (hB < 32 && (1ull << hB) < idx->n) ++hB;
-  hB = std::max(hB, hbits);
+  DgIndex::Schedule sched = schedule_of(idx, trav, lcap, filt, maxL);
+  sched.wpb = 0;
 
   // scratch layout: [0, 256) work counter | filter ops | offsets | pool | beams | per-query k
   auto up16 = [](size_t x) { return (x + 15) & ~(size_t)15; };
@@ -1219,8 +1234,6 @@ extern "C" DgStatus dg_search_batch_static(DgIndex *idx, const DgSearchParams *p
   a.k = p->k;
   a.L = p->beam_width;
   a.rerank = p->rerank_size;
-  a.hbits = hbits;
-  a.hB = hB;
   // every call reuses the array: the counter must start at zero again
   DG_CUDA(cudaMemsetAsync(scratch, 0, 4, st));
   a.counter = reinterpret_cast<uint32_t *>(scratch);
@@ -1257,8 +1270,10 @@ extern "C" DgStatus dg_search_batch_static(DgIndex *idx, const DgSearchParams *p
   if (trav == TRAV_F32) lpr = 8;
   else if (trav == TRAV_BF16 || trav == TRAV_F16) lpr = lanes_per_row(idx->dpad / 8);
   else if (trav == TRAV_INT8) lpr = lanes_per_row(idx->code_stride / 16);
-  const SearchPlan P = plan_search(idx, trav, lcap, filt, need, search_k, reranked, hbits, 0, nq);
+  const SearchPlan P = plan_search(idx, trav, lcap, filt, need, search_k, reranked, sched, nq);
   a.limit_smem = P.limit_smem;
+  a.hbits = P.hbits;
+  a.hB = P.hB;
   LaunchInfo info;
   switch (trav) {
     case TRAV_F32: s = launch_search_f32(a, P.Ly, met, lpr, P.cta, P.tc, filt, st, &info); break;

@@ -48,6 +48,7 @@ struct DgIndex {
   // finely when each query holds a large state).
   struct Schedule {
     uint32_t hbits = 0, order = 0, occ_pct = 100, wpb = 4;  // wpb: warps (queries in flight) per CTA
+    bool chosen = false;      // the table size was tuned or given: a search does not adapt it
   };
   std::map<uint32_t, Schedule> tuned;
   bool forcing = false;   // the autotuner pins `force` while it times a candidate

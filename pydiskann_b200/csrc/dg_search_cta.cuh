@@ -339,15 +339,17 @@ __device__ inline void search_cta(const SearchArgs &a, uint32_t q, uint8_t *sm, 
   }
 
   // a result must be live (UnifiedView::is_live, src/incremental.rs:463-470) and match
-  // Rows of up to four label fields are loaded ahead of the distances (l).
-  const bool few = labeled && a.nf <= 4;
-  auto allow = [&](uint32_t id, const uint64_t (&l)[4]) -> bool {
+  auto allow = [&](uint32_t id) -> bool {
     if (a.tomb && ((__ldg(a.tomb + (id >> 5)) >> (id & 31)) & 1u)) return false;
-    if (few)
-      return filter_eval_by(qc.fops, qc.fnops, a.fpool, a.nf, [&](uint32_t f) {
-        return f == 0 ? l[0] : f == 1 ? l[1] : f == 2 ? l[2] : l[3];
-      });
-    return !labeled || filter_eval(qc.fops, qc.fnops, a.fpool, a.labels + (size_t)id * a.nf, a.nf);
+    if (!labeled) return true;
+    const uint64_t *row = a.labels + (size_t)id * a.nf;
+    if (a.nf > 4) return filter_eval(qc.fops, qc.fnops, a.fpool, row, a.nf);
+    uint64_t l[4];  // the whole row at once
+#pragma unroll
+    for (uint32_t f = 0; f < 4; ++f) l[f] = f < a.nf ? __ldg(row + f) : 0ull;
+    return filter_eval_by(qc.fops, qc.fnops, a.fpool, a.nf, [&](uint32_t f) {
+      return f == 0 ? l[0] : f == 1 ? l[1] : f == 2 ? l[2] : l[3];
+    });
   };
 
   // ---- seeds: the medoid, and the delta layer's entry point of a base + delta
@@ -389,19 +391,16 @@ __device__ inline void search_cta(const SearchArgs &a, uint32_t q, uint8_t *sm, 
     for (int g0 = warp * share; g0 < g1; g0 += B) {
       const int cnt = min(B, g1 - g0);
       const uint32_t cand = lane < cnt ? stage[g0 + lane] : DG_PAD;
-      uint64_t lab[4];
-      if (FILT && few) {
-#pragma unroll
-        for (uint32_t f = 0; f < 4; ++f)
-          lab[f] = lane < cnt && f < a.nf ? __ldg(a.labels + (size_t)cand * a.nf + f) : 0ull;
-      }
+      // the label row is on its way under the distances
+      if (FILT && labeled && lane < cnt)
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(a.labels + (size_t)cand * a.nf));
       float d = cta_distance<B, TRAV, MET, LPR, TC>(a, sm, Ly, cand, cnt, lane, qq);
       if (TRAV != TRAV_F32 && a.code_limit < a.n && lane < cnt && cand >= a.code_limit)
         d = exact_row_distance<MET>(a, qs, cand, qq);
       const uint64_t key = lane < cnt ? make_key(d, cand) : kKeyInvalid;
       cta_survive<NW>(lists[0], key, key < thr, ctl + CTL_CNT, lane);
       if (FILT && filtered)
-        cta_survive<NW>(lists[1], key, lane < cnt && key < rthr && allow(cand, lab), ctl + CTL_CNTR, lane);
+        cta_survive<NW>(lists[1], key, lane < cnt && key < rthr && allow(cand), ctl + CTL_CNTR, lane);
     }
     cta_sync<NW>();  // every warp's survivors are in place
     const int s[2] = {(int)ctl[CTL_CNT], FILT ? (int)ctl[CTL_CNTR] : 0};

@@ -442,7 +442,7 @@ static uint64_t working_need(const DgIndex *idx, uint32_t maxL, uint32_t k, uint
   if (any_filter) need = std::max<uint64_t>({(uint64_t)maxL * 4, (uint64_t)k * 10, search_k});
   else if (tombed)
     need = std::max<uint64_t>({(uint64_t)maxL * 2, search_k + std::min<uint64_t>(idx->ntomb, maxL), search_k});
-  // two entry points run in the general kernel (the 64-entry register-list
+  // two entry points run in the CTA-per-query kernel (the 64-entry register-list
   // kernel seeds the medoid only), which a capacity above 64 selects
   if (idx->seed2 != DG_PAD) need = std::max<uint64_t>(need, 65);
   *filt = any_filter || tombed;

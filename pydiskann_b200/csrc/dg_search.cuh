@@ -1,14 +1,15 @@
-// dg_search.cuh -- warp-per-query best-first beam search (sm_100a).
+// dg_search.cuh -- shared parts of the best-first beam search (sm_100a).
 //
-// Restates beam_search (diskann-rs src/lib.rs:198-303) for one query per warp:
-//   * the working set `w` is a sorted shared-memory array of 64-bit keys
-//     ((distance, id) order, bit 0 = "expanded");  the reference's frontier
-//     min-heap is the first unexpanded entry of that array, because an entry
-//     the reference evicts from `w` is never smaller than the current worst of
-//     `w` and therefore only ever ends the search;
+// Restates beam_search (diskann-rs src/lib.rs:198-303); the kernels are in
+// dg_search_kernel.cuh (one warp per query, the list in registers) and
+// dg_search_cta.cuh (one CTA per query, the list in shared memory):
+//   * the working set `w` is a sorted array of 64-bit keys ((distance, id)
+//     order, bit 0 = "expanded");  the reference's frontier min-heap is the
+//     first unexpanded entry of that array, because an entry the reference
+//     evicts from `w` is never smaller than the current worst of `w` and
+//     therefore only ever ends the search;
 //   * one expansion gathers the adjacency row, drops visited ids, computes all
-//     new distances in one batch and merges them into `w` with a warp-wide
-//     bitonic sort and a merge-path scatter.  Processing a row as one batch
+//     new distances and merges them into `w`.  Processing a row as one batch
 //     keeps exactly the L smallest (distance, id) pairs, which is what the
 //     reference's sequential insert-if-smaller loop keeps;
 //   * the visited set is a small exact-tag table in shared memory (struct
@@ -22,7 +23,7 @@
 //   * quantized search (src/quantized.rs:68-124) traverses on codes, then
 //     reranks the first max(rerank, k) entries with exact FP32 distances in
 //     their code-distance order (a stable sort by exact distance).
-// Warps take queries from a global counter, so uneven beams, k and filters
+// Queries are taken from a global counter, so uneven beams, k and filters
 // balance across the persistent grid.
 #pragma once
 #include "dg_common.cuh"

@@ -12,14 +12,14 @@
 // L smallest (distance, id) pairs after every expansion, the same visited
 // table contents (so the same counts) and the same stopping rules.
 //
-// What bounds it is the chain of one expansion (cycles on one 8-warp CTA of
-// the 100k x 128 FP32 search, beam 128: neighbour list and visited test 1350,
-// row distances 2000, merge 840, selection 310), not bandwidth (DRAM 4 %, issue
-// 35 % in a filtered batch).  Against the kernel before it (one warp per query,
-// two copies of the list in shared memory, merged entry by entry): one query
-// of that search 547 -> 405 us; 4000 768-d int8 cosine queries with beams up to
-// 256 17.2 -> 7.9 ms; 5000 PQ queries, beam 128, 7.75 -> 3.27 ms; 500 filtered
-// queries, k = 100, 15.7 -> 8.2 ms; 2000 filtered queries, k = 10, 5.85 -> 4.3 ms.
+// What bounds it is the chain of one expansion, not bandwidth (cycles on one
+// 8-warp CTA of the 100k x 128 FP32 search, beam 128: neighbour list and visited
+// test 1120, row distances 1160, merge 720, selection 300; DRAM 6 %, issue 35 %
+// in a filtered batch).  Against the kernel before it (one warp per query, two
+// copies of the list in shared memory, merged entry by entry): one query of that
+// search 547 -> 345 us; 4000 768-d int8 cosine queries with beams up to 256 16.9
+// -> 6.7 ms; 5000 PQ queries, beam 128, 7.7 -> 2.6 ms; 500 filtered queries,
+// k = 100, 16.4 -> 7.9 ms; 2000 filtered queries, k = 10, 5.9 -> 4.1 ms.
 #pragma once
 #include "dg_search_kernel.cuh"
 

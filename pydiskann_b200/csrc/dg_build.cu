@@ -98,10 +98,12 @@ __global__ void k_pq_encode(const float *v, uint64_t n, uint32_t dpad, uint32_t 
 }
 
 // The same for the usual widths: the subspace's codebook sits in shared
-// memory, two centroids interleaved, a thread holds two sub-vectors in
-// registers, and each packed instruction serves two centroids (a subtraction,
-// a multiplication and an addition per coordinate, each rounded once, in
-// coordinate order: the same bits).  Bound by FP32 issue; the kernel above
+// memory, two centroids interleaved, and a thread holds two sub-vectors in
+// registers, so that each load of a centroid pair serves four distances (a
+// subtraction, a multiplication and an addition per coordinate, each rounded
+// once, in coordinate order: the same bits.  Packed two-wide forms were
+// contracted to FMAs, which changed one code in eight million).  Bound by FP32
+// issue; the kernel above
 // re-reads the sub-vector and the centroid for every term (200k rows, M = 16,
 // K = 256, 8 wide: 24 ms).
 template <int DS>
@@ -117,7 +119,6 @@ __global__ void __launch_bounds__(256) k_pq_nearest(const float *__restrict__ v,
     cs[e] = make_float2(p[0], c + 1 < K ? p[DS] : inf);  // (an infinite distance is never the smallest)
   }
   __syncthreads();
-  const float2 neg1 = make_float2(-1.0f, -1.0f);
   const uint64_t step = (uint64_t)gridDim.x * blockDim.x;
   for (uint64_t i0 = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i0 < n; i0 += 2 * step) {
     const uint64_t i1 = i0 + step < n ? i0 + step : i0;
@@ -143,10 +144,12 @@ __global__ void __launch_bounds__(256) k_pq_nearest(const float *__restrict__ v,
 #pragma unroll
       for (int j = 0; j < DS; ++j) {
         const float2 cv = cs[c * DS + j];
-        const float2 t0 = __ffma2_rn(cv, neg1, make_float2(a[j], a[j]));  // x - c, one rounding
-        const float2 t1 = __ffma2_rn(cv, neg1, make_float2(b[j], b[j]));
-        s0 = __fadd2_rn(s0, __fmul2_rn(t0, t0));
-        s1 = __fadd2_rn(s1, __fmul2_rn(t1, t1));
+        const float t0 = __fsub_rn(a[j], cv.x), t1 = __fsub_rn(a[j], cv.y);
+        const float u0 = __fsub_rn(b[j], cv.x), u1 = __fsub_rn(b[j], cv.y);
+        s0.x = __fadd_rn(s0.x, __fmul_rn(t0, t0));
+        s0.y = __fadd_rn(s0.y, __fmul_rn(t1, t1));
+        s1.x = __fadd_rn(s1.x, __fmul_rn(u0, u0));
+        s1.y = __fadd_rn(s1.y, __fmul_rn(u1, u1));
       }
       if (s0.x < best0) { best0 = s0.x; c0 = 2 * c; }
       if (s0.y < best0) { best0 = s0.y; c0 = 2 * c + 1; }

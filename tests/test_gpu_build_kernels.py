@@ -44,6 +44,19 @@ def test_pq_encode_widths(oracle, ds, K):
     assert np.array_equal(dg.pq_encode(X, cb), oracle.pq_encode(X, cb))
 
 
+@pytest.mark.parametrize("ds", [2, 4, 6, 8, 10, 12, 16])
+def test_pq_encode_near_ties(oracle, ds):
+    """Rows halfway between two centroids of inexact values: which one is nearer is decided by the
+    rounding of every product and sum, so a contracted one shows."""
+    M, K, n = 2, 64, 30_000
+    rng = np.random.default_rng(ds)
+    cb = (rng.standard_normal((M, K, ds)) * 50).astype(np.float32)
+    a, b = rng.integers(0, K, (2, n, M))
+    m = np.arange(M)
+    X = ((cb[m, a] + cb[m, b]) * np.float32(0.5)).reshape(n, M * ds)
+    assert np.array_equal(dg.pq_encode(X, cb), oracle.pq_encode(X, cb))
+
+
 @pytest.mark.parametrize("n,ds,K", [(40, 4, 64), (1025, 8, 32), (5000, 3, 256), (2600, 40, 16)])
 def test_pq_train_blocks(oracle, n, ds, K):
     X = synth.mixture(n, 2 * ds, 8, seed=6)

@@ -1227,7 +1227,9 @@ __global__ void __launch_bounds__(256, 3) k_pm_scan_postings(SpfArgs a, const ui
         }
       }
     }
-    __syncwarp();
+    // a live posting may hold no entry: no tile, and no barrier but this one
+    // between warp 0's set-up of `state` and the other warps' reads of it
+    __syncthreads();
 #pragma unroll 1
     for (uint32_t j = warp; j < m; j += 8) {
       const int size = (int)(state[j] >> 1);

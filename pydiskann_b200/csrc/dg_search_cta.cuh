@@ -72,7 +72,10 @@ __device__ __forceinline__ void cta_sync() {
 }
 template <int NW>
 __device__ __forceinline__ int cta_sync_count(bool v) {
-  return NW == 1 ? __popc(__ballot_sync(kFull, v)) : __syncthreads_count(v);
+  if (NW != 1) return __syncthreads_count(v);
+  const int n = __popc(__ballot_sync(kFull, v));
+  __syncwarp();  // (a ballot orders no memory)
+  return n;
 }
 
 // Candidates a warp takes at a time.  8 long rows of an eighth, or 16, keep a quarter (an eighth, a half) of

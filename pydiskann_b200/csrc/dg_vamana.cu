@@ -588,6 +588,7 @@ __global__ void __launch_bounds__(kPruneThreads, 2) k_prune_small(PruneArgs a) {
       return j < staged ? tile + (size_t)j * ts : reinterpret_cast<const uint4 *>(rows) + (size_t)key_id(K[j]) * chunks;
     };
     if (TC) {
+      const uint32_t quad = 0xfu << (lane & 28);  // (quads leave the loop at different times)
       for (int j = 8 * warp + (lane >> 2); j < m; j += 64) {  // four lanes per row
         const uint4 *x = row_of(j);
         float s2 = 0.0f;
@@ -597,8 +598,8 @@ __global__ void __launch_bounds__(kPruneThreads, 2) k_prune_small(PruneArgs a) {
 #pragma unroll
           for (int e = 0; e < 8; ++e) s2 = fmaf(v[e], v[e], s2);
         }
-        s2 += __shfl_xor_sync(__activemask(), s2, 1);
-        s2 += __shfl_xor_sync(__activemask(), s2, 2);
+        s2 += __shfl_xor_sync(quad, s2, 1);
+        s2 += __shfl_xor_sync(quad, s2, 2);
         if ((lane & 3) == 0) P.norm[j] = (int)s2;
       }
     }

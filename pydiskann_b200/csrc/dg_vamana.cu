@@ -765,6 +765,7 @@ __global__ void __launch_bounds__(kPruneThreads, 2) k_prune_small(PruneArgs a) {
         if (ok && at < a.R) P.out[at] = key_id(K[i]);
         np = min(a.R, np + (uint32_t)__popc(mk));
       }
+      __syncwarp();  // the entries above are other lanes'
       for (uint32_t j = lane; j < a.R; j += 32) a.out[u * a.R + j] = j < np ? P.out[j] : DG_PAD;
     }
     __syncthreads();

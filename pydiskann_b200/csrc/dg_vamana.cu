@@ -456,14 +456,14 @@ __host__ __device__ inline uint32_t prune_stride16(uint32_t chunks, bool tc) {
 // and with the walk's thresholds 1, 1.2, 1.44, ... up to alpha, so the
 // approximate quotient (2 ulp for |d| in [2^-126, 2^126]) stands in for the
 // rounded one wherever both lie on the same side of each of them; within 8 ulp
-// of one, and for extreme divisors, the rounded quotient is taken.  (The
-// rounded division is a call of some 280 cycles here; it was two thirds of a
-// pruned node's time.)
+// of one, for extreme divisors, and for alpha above 8 (more than 12
+// thresholds), the rounded quotient is taken.  (The rounded division is a call
+// of some 280 cycles here; it was two thirds of a pruned node's time.)
 __device__ __forceinline__ float prune_ratio(float kd, float d, float alpha) {
   const float r = __fdividef(kd, d), ad = fabsf(d);
   bool exact = !(ad > 1e-30f && ad < 1e30f) || fabsf(r - 1.0f) <= 1e-6f || fabsf(r - 1.2f) <= 1.2e-6f ||
-               fabsf(r - alpha) <= 1e-6f * alpha;
-  if (alpha > 1.2f)
+               fabsf(r - alpha) <= 1e-6f * alpha || alpha > 8.0f;
+  if (alpha > 1.2f && alpha <= 8.0f)
     for (float t = 1.2f; t <= alpha; t = __fmul_rn(t, 1.2f)) exact |= fabsf(r - t) <= 1e-6f * t;
   if (!exact) return r;
   return d == 0.0f ? __int_as_float(0x7f800000) : __fdiv_rn(kd, d);
@@ -1069,6 +1069,10 @@ extern "C" DgStatus dg_build_vamana(const float *X, uint64_t n, uint32_t dim, in
   if (build_beam == 0 || build_beam > 1024) return fail(DG_EINVAL, "build_beam_width must be in [1, 1024]");
   if (medoid >= n) return fail(DG_EINVAL, "medoid out of range");
   if (metric < DG_L2SQ || metric > DG_DOT) return fail(DG_EINVAL, "unknown metric");
+  // the relaxed passes multiply their threshold until it exceeds alpha, which it
+  // never does when both are infinite; the largest float keeps the same entries
+  // (what the pass at infinity would add, the fill adds in the same order)
+  alpha = std::min(alpha, 3.402823466e38f);
   DG_CUDA(cudaSetDevice(device));
   cudaStream_t st;
   DG_CUDA(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));

@@ -1098,7 +1098,7 @@ __global__ void __launch_bounds__(256, 3) k_pm_scan_postings(SpfArgs a, const ui
         s2 += __shfl_xor_sync(kFull, s2, 1);
         s2 += __shfl_xor_sync(kFull, s2, 2);
         if (c0 == 0) {
-          xn[r] = s2;  // (exact where it is used: tensor-core tiles)
+          xn[r] = s2;  // (stands where any order of the sum is exact)
           uint32_t id = DG_PAD;
           if (r < ne) {
             id = __ldg(a.ids + b * a.cap + e0 + r);
@@ -1111,7 +1111,27 @@ __global__ void __launch_bounds__(256, 3) k_pm_scan_postings(SpfArgs a, const ui
       }
       const bool tbad = __syncthreads_or(bad);
       // (an inexact query makes s_qmax infinite; the candidates overlay the f32 tile)
-      const bool tc = !tbad && (float)a.d * s_qmax * __uint_as_float(s_tmax) < kPmExactSum;
+      const float tmax = __uint_as_float(s_tmax);
+      const bool tc = !tbad && (float)a.d * s_qmax * tmax < kPmExactSum;
+      // entry norms where the sum may round: one order for both kinds of tile, so
+      // that a distance does not depend on the queries it is scored beside.  Four
+      // lanes per row (8 rows per warp pass), interleaved coordinates, so a
+      // quarter warp reads one row's consecutive words.
+      auto entry_norms = [&](auto at) {
+        for (uint32_t r0 = 8u * warp; r0 < ne; r0 += 8u * 8u) {
+          const uint32_t r = r0 + (lane >> 2);
+          float s2 = 0.0f;
+          if (r < ne)
+            for (uint32_t i = lane & 3; i < a.d; i += 4) s2 = fmaf(at(r, i), at(r, i), s2);
+          s2 += __shfl_xor_sync(kFull, s2, 1);
+          s2 += __shfl_xor_sync(kFull, s2, 2);
+          if (r < ne && (lane & 3) == 0) xn[r] = s2;
+        }
+      };
+      if (tc && (float)a.d * tmax * tmax >= kPmExactSum) {  // (the FP16 rows hold the values exactly)
+        entry_norms([&](uint32_t r, uint32_t i) { return __half2float(__ushort_as_half(th[r * ks + i])); });
+        __syncthreads();
+      }
       if (tc) {
         // warp w: entries 16 (w % 4) .. +15 against queries 16 (w / 4) .. +15
         const uint32_t e16 = 16u * (warp & 3), q16 = 16u * (warp >> 2);
@@ -1153,17 +1173,7 @@ __global__ void __launch_bounds__(256, 3) k_pm_scan_postings(SpfArgs a, const ui
         }
         if (!have_q) stage_queries();
         __syncthreads();
-        // entry norms: four lanes per row (8 rows per warp pass), interleaved
-        // coordinates, so a quarter warp reads one row's consecutive words
-        for (uint32_t r0 = 8u * warp; r0 < ne; r0 += 8u * 8u) {
-          const uint32_t r = r0 + (lane >> 2);
-          float s2 = 0.0f;
-          if (r < ne)
-            for (uint32_t i = lane & 3; i < a.d; i += 4) s2 = fmaf(tile[r * dt + i], tile[r * dt + i], s2);
-          s2 += __shfl_xor_sync(kFull, s2, 1);
-          s2 += __shfl_xor_sync(kFull, s2, 2);
-          if (r < ne && (lane & 3) == 0) xn[r] = s2;
-        }
+        entry_norms([&](uint32_t r, uint32_t i) { return tile[r * dt + i]; });
         float acc[4][2];
 #pragma unroll
         for (int u = 0; u < 4; ++u) acc[u][0] = acc[u][1] = 0.0f;

@@ -531,7 +531,9 @@ static uint32_t traversal_row_bytes(const DgIndex *idx, int trav) {
 // half the default visited table: a forgotten id only costs its distance
 // again (5000 PQ queries, beam 128, 2^11 -> 2^10 words: 3215 -> 2630 us; 4000
 // 768-d int8 cosine queries, beams up to 256, 2^12 -> 2^11: 7926 -> 6757 us;
-// one step more: 2618 and 7770).
+// one step more: 2618 and 7770).  A call that returns the counts of evaluated
+// ids keeps the whole table, so that a query's counts do not depend on how many
+// others are searched with it.
 struct SearchPlan {
   WarpLayout Ly;
   uint32_t hbits, hB;   // visited table: log2 words, id bits
@@ -540,7 +542,7 @@ struct SearchPlan {
   uint32_t limit_smem;  // what decides whether the search is accepted, whichever kernel runs
 };
 static SearchPlan plan_search(const DgIndex *idx, int trav, int lcap, bool filt, uint64_t need, uint32_t search_k,
-                              bool reranked, const DgIndex::Schedule &sc, uint32_t nq) {
+                              bool reranked, const DgIndex::Schedule &sc, uint32_t nq, bool counted) {
   SearchPlan P;
   P.hbits = sc.hbits;
   const bool decode = (trav == TRAV_RABITQ || trav == TRAV_INT8) && met_kind(idx->metric) != MET_L2;
@@ -559,7 +561,7 @@ static SearchPlan plan_search(const DgIndex *idx, int trav, int lcap, bool filt,
     return 227u * 1024u / (P.Ly.total + 1024u);
   };
   uint32_t room = fit(P.hbits);
-  if (!sc.chosen && nq > 5 * sms && room < 12 && P.hbits > 10) room = fit(--P.hbits);
+  if (!sc.chosen && !counted && nq > 5 * sms && room < 12 && P.hbits > 10) room = fit(--P.hbits);
   // traversals whose lone warp takes 32 candidates at a time (cta_batch)
   const bool short_rows = trav == TRAV_INT8 || trav == TRAV_FP8 || trav == TRAV_PQ || trav == TRAV_RABITQ ||
                           ((trav == TRAV_BF16 || trav == TRAV_F16) && lanes_per_row(idx->dpad / 8) != 8);
@@ -841,7 +843,8 @@ DgStatus dg_search_batch(DgIndex *idx, const DgSearchParams *p, const float *que
       aa.perm = perm + q0;
     }
     DG_CUDA(cudaMemsetAsync(aa.counter, 0, 4, ss));
-    const SearchPlan P = plan_search(idx, trav, lcap, filt, need, search_k, reranked, sched, nq);
+    const SearchPlan P =
+        plan_search(idx, trav, lcap, filt, need, search_k, reranked, sched, nq, a.out_stats != nullptr);
     aa.limit_smem = P.limit_smem;
     aa.hbits = P.hbits;
     aa.hB = P.hB;
@@ -1270,7 +1273,7 @@ extern "C" DgStatus dg_search_batch_static(DgIndex *idx, const DgSearchParams *p
   if (trav == TRAV_F32) lpr = 8;
   else if (trav == TRAV_BF16 || trav == TRAV_F16) lpr = lanes_per_row(idx->dpad / 8);
   else if (trav == TRAV_INT8) lpr = lanes_per_row(idx->code_stride / 16);
-  const SearchPlan P = plan_search(idx, trav, lcap, filt, need, search_k, reranked, sched, nq);
+  const SearchPlan P = plan_search(idx, trav, lcap, filt, need, search_k, reranked, sched, nq, false);
   a.limit_smem = P.limit_smem;
   a.hbits = P.hbits;
   a.hB = P.hB;

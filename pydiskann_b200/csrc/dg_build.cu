@@ -714,8 +714,14 @@ __global__ void __launch_bounds__(128) k_knn_merge(const uint64_t *part, const u
   }
 }
 
-// Launches the tiled kNN: the rows are cut into the number of slices that
-// leaves the fewest tiles to the busiest of the 2 CTAs per SM.
+// Launches the tiled kNN: the rows are cut into the number of slices that costs
+// the busiest of the resident CTAs (2 per SM for k up to 64, 1 above, whose lists
+// take 128 KB) least, as far as the slices' lists stay within kKnnPartBytes.  A
+// tile takes about 5.5 + 0.11 dim us; filling the lists of a slice's 64 queries
+// 12 k us more, whatever its length, so that long lists want few slices (100k
+// rows, 10k queries, k = 100, 16 / 3 slices: 8-d 51.6 / 30.5 ms, 32-d 51.4 / 31.9;
+// 20k x 128-d queries, k = 64, 16 / 4: 85.9 / 61.5).
+constexpr size_t kKnnPartBytes = (size_t)256 << 20;
 static DgStatus knn_tiled(const float *v, uint64_t n, uint32_t dim, uint32_t dpad, const float *q, uint32_t nq,
                           uint32_t k, int metric, uint32_t *oi, float *od, cudaStream_t st) {
   int dev = 0, sms = 0;
@@ -724,10 +730,19 @@ static DgStatus knn_tiled(const float *v, uint64_t n, uint32_t dim, uint32_t dpa
   uint32_t kcap = 16;
   while (kcap < k) kcap <<= 1;
   const size_t smem = align16(2 * kKnnJ * kKnnS * 8 + kKnnT * (kKnnT + 1) * 4) + 8 * 32 * 8 + (size_t)kKnnT * 2 * kcap * 8;
-  const uint64_t qb = (nq + kKnnT - 1) / kKnnT, tiles = (n + kKnnT - 1) / kKnnT, slots = 2ull * sms;
-  uint64_t best = ~0ull, slices = 1;
-  for (uint64_t s = 1; s <= std::min<uint64_t>(tiles, 4 * slots); ++s) {
-    const uint64_t cost = ((qb * s + slots - 1) / slots) * ((tiles + s - 1) / s + 2);
+  const bool l2 = metric == DG_L2SQ || metric == DG_L2;
+  auto kern = l2 ? k_knn_tiled<true> : k_knn_tiled<false>;
+  int per_sm = 0;
+  DG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  DG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 256, smem));
+  const uint64_t qb = (nq + kKnnT - 1) / kKnnT, tiles = (n + kKnnT - 1) / kKnnT;
+  const uint64_t slots = (uint64_t)std::max(1, per_sm) * sms;
+  const uint64_t most = std::min({tiles, 4 * slots, (uint64_t)(kKnnPartBytes / std::max<size_t>((size_t)nq * k * 8, 1))});
+  const double fill = 12.0 * k / (5.5 + 0.11 * dim);  // in tiles
+  double best = 1e300;
+  uint64_t slices = 1;
+  for (uint64_t s = 1; s <= most; ++s) {
+    const double cost = (double)((qb * s + slots - 1) / slots) * ((double)((tiles + s - 1) / s + 2) + fill);
     if (cost < best) {
       best = cost;
       slices = s;
@@ -744,11 +759,8 @@ static DgStatus knn_tiled(const float *v, uint64_t n, uint32_t dim, uint32_t dpa
       if (p) cudaFreeAsync(p, st);
     return fail(DG_ENOMEM, "exact knn staging");
   }
-  const bool l2 = metric == DG_L2SQ || metric == DG_L2;
-  auto kern = l2 ? k_knn_tiled<true> : k_knn_tiled<false>;
   DgStatus s = DG_OK;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e == cudaSuccess) e = cudaMemsetAsync(thr, 0xff, (size_t)nq * 4, st);
+  cudaError_t e = cudaMemsetAsync(thr, 0xff, (size_t)nq * 4, st);
   if (e == cudaSuccess) {
     kern<<<dim3((unsigned)qb, (unsigned)slices), 256, smem, st>>>(v, n, dim, dpad, q, nq, k, metric, kcap, rows, thr,
                                                                   part, pc);

@@ -778,6 +778,21 @@ static DgStatus knn_tiled(const float *v, uint64_t n, uint32_t dim, uint32_t dpa
   return s;
 }
 
+// Whether the tiled kernel takes a call (the same results either way).  Its
+// tiles halve and better the FP64 time of a pair, 0.4 ps x dim on the whole GPU;
+// its slices and 64-query barriers make a list entry dearer, by 22 ns at 100k rows
+// and about in proportion to the root of their number.  So few coordinates, few
+// rows and long lists favour one list per query, once there are enough queries to
+// fill the GPU that way (ms, one list / tiles; 10k queries x 100k rows: 8-d, k = 10
+// 10.0 / 10.2, k = 100 15.6 / 31.4; 32-d, k = 32 24.8 / 19.4, k = 100 28.1 / 33.4;
+// 128-d, k = 128 86 / 53; 10k rows: 32-d, k = 10 3.3 / 3.5, k = 100 4.9 / 10.7; 1000
+// queries x 100k rows: 8-d, k = 100 6.9 / 6.8, 32-d 10.3 / 7.7).  Lists above
+// kKnnTileK do not fit a tile CTA; above 1024 coordinates tiles always win.
+static bool knn_by_tiles(uint64_t n, uint32_t dim, uint32_t nq, uint32_t k) {
+  if (k > (uint32_t)kKnnTileK) return false;
+  return nq <= 1024 || dim > 1024 || 200.0 * k <= dim * std::sqrt((double)n);
+}
+
 // ------------------------------------------------------------ PQ training
 // ProductQuantizer::train (src/pq.rs:51-119): per subspace, k-means++ seeding
 // then Lloyd iterations; empty clusters restart from a random training point.
@@ -1217,9 +1232,9 @@ DgStatus dg_exact_knn(const float *X, uint64_t n, uint32_t dim, const float *Q, 
     s = fail(DG_ENOMEM, "exact knn staging");
   if (s == DG_OK) s = upload_rows_f32(X, n, dim, dpad, v, st);
   if (s == DG_OK) cudaMemcpyAsync(q, Q, (size_t)nq * dim * 4, cudaMemcpyHostToDevice, st);
-  if (s == DG_OK && k <= (uint32_t)kKnnTileK) {
+  if (s == DG_OK && knn_by_tiles(n, dim, nq, k)) {
     s = knn_tiled(v, n, dim, dpad, q, nq, k, metric, oi, od, st);
-  } else if (s == DG_OK) {  // longer lists than a 64-query CTA can hold: 8 queries per CTA
+  } else if (s == DG_OK) {  // 8 queries per CTA, one list each
     uint32_t kcap = 32;
     while (kcap < k) kcap <<= 1;
     const size_t smem = align16((32 * (dim + 1) + kKnnWarps * dim) * 4) + (size_t)kKnnWarps * (2 * kcap + 32) * 8;

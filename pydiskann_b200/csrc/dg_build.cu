@@ -757,6 +757,7 @@ static DgStatus knn_tiled(const float *v, uint64_t n, uint32_t dim, uint32_t dpa
       cudaMallocAsync(&part, (size_t)slices * nq * k * 8, st) != cudaSuccess) {
     for (void *p : {(void *)thr, (void *)pc, (void *)part})
       if (p) cudaFreeAsync(p, st);
+    cudaGetLastError();
     return fail(DG_ENOMEM, "exact knn staging");
   }
   DgStatus s = DG_OK;
@@ -1232,9 +1233,12 @@ DgStatus dg_exact_knn(const float *X, uint64_t n, uint32_t dim, const float *Q, 
     s = fail(DG_ENOMEM, "exact knn staging");
   if (s == DG_OK) s = upload_rows_f32(X, n, dim, dpad, v, st);
   if (s == DG_OK) cudaMemcpyAsync(q, Q, (size_t)nq * dim * 4, cudaMemcpyHostToDevice, st);
-  if (s == DG_OK && knn_by_tiles(n, dim, nq, k)) {
-    s = knn_tiled(v, n, dim, dpad, q, nq, k, metric, oi, od, st);
-  } else if (s == DG_OK) {  // 8 queries per CTA, one list each
+  bool tiled = s == DG_OK && knn_by_tiles(n, dim, nq, k);
+  if (tiled && (s = knn_tiled(v, n, dim, dpad, q, nq, k, metric, oi, od, st)) == DG_ENOMEM) {
+    tiled = false;  // the partial lists do not fit beside the rows: the other kernel needs none
+    s = DG_OK;
+  }
+  if (s == DG_OK && !tiled) {  // 8 queries per CTA, one list each
     uint32_t kcap = 32;
     while (kcap < k) kcap <<= 1;
     const size_t smem = align16((32 * (dim + 1) + kKnnWarps * dim) * 4) + (size_t)kKnnWarps * (2 * kcap + 32) * 8;

@@ -68,6 +68,8 @@ __global__ void k_pad_rows(const float *__restrict__ src, uint64_t n, uint32_t d
 DgStatus upload_rows_f32(const float *host, uint64_t n, uint32_t d, uint32_t dpad, float *dev, cudaStream_t st,
                          const uint64_t *rows) {
   const size_t row = (size_t)d * sizeof(float);
+  int device = 0;
+  DG_CUDA(cudaGetDevice(&device));
   UploadPool &pool = upload_pool();
   std::unique_lock<std::mutex> lk(pool.mu, std::defer_lock);
   bool staged = n * row >= kUpMin && row <= kUpPiece;
@@ -81,6 +83,13 @@ DgStatus upload_rows_f32(const float *host, uint64_t n, uint32_t d, uint32_t dpa
       cudaHostAlloc((void **)&pool.mem, kUpThreads * kUpBufs * kUpPiece, cudaHostAllocPortable) != cudaSuccess) {
     cudaGetLastError();
     pool.mem = nullptr;
+    staged = false;
+  }
+  uint8_t *landing = nullptr;  // padded rows: pieces land here and are spread by k_pad_rows, in stream order
+  if (staged && d != dpad &&
+      cudaMallocAsync((void **)&landing, kUpThreads * kUpBufs * kUpPiece, st) != cudaSuccess) {
+    cudaGetLastError();  // (a device full but for the rows: the strided copy needs no room)
+    landing = nullptr;
     staged = false;
   }
   if (!staged) {
@@ -99,10 +108,6 @@ DgStatus upload_rows_f32(const float *host, uint64_t n, uint32_t d, uint32_t dpa
     if (rows) DG_CUDA(cudaStreamSynchronize(st));  // the gathered copy goes now
     return DG_OK;
   }
-  int device = 0;
-  DG_CUDA(cudaGetDevice(&device));
-  uint8_t *landing = nullptr;  // padded rows: pieces land here and are spread by k_pad_rows, in stream order
-  if (d != dpad) DG_CUDA(cudaMallocAsync((void **)&landing, kUpThreads * kUpBufs * kUpPiece, st));
   const uint64_t per = kUpPiece / row, pieces = (n + per - 1) / per;
   cudaError_t err[kUpThreads] = {};
   auto work = [&](int t) {

@@ -913,14 +913,19 @@ static DgStatus run_build(const BuildArgs &base, float *vf, uint16_t *vb, bool t
     return DG_OK;
   };
   // search kernel geometry
-  const uint32_t hbits = base.Lb <= 64 ? 10 : base.Lb <= 128 ? 11 : 12;
+  // (a larger visited table for beams above 128 leaves two CTAs per SM instead of
+  // four or five; a forgotten id costs its distance again.  Searches of 20k real
+  // rows x 128, R = 64, 2^12 / 2^11 words: beam 200 121 / 58 ms, 256 149 / 84, 400
+  // 249 / 141, 800 517 / 403; integer rows, beam 256, 77 / 46)
+  const uint32_t hbits = base.Lb <= 64 ? 10 : 11;
   const BuildLayout Ly = build_layout(base.Lb, R, hbits, dpad, tc);
   void (*sk)(BuildArgs, BuildLayout) = k_build_search<ELEM, MET, LPR, false>;
   if constexpr (ELEM == 1 && MET != MET_COS)
     if (tc) sk = k_build_search<ELEM, MET, LPR, true>;
   // (accepted or refused by the state of a two-list search, as ever)
   const uint32_t lcap = base.Lb <= 64 ? 64 : base.Lb <= 256 ? 256 : 1024;
-  const WarpLayout limit = warp_layout(ELEM == 1 ? TRAV_BF16 : TRAV_F32, lcap, false, hbits, dpad, 0, 0, 0);
+  const WarpLayout limit = warp_layout(ELEM == 1 ? TRAV_BF16 : TRAV_F32, lcap, false, base.Lb <= 128 ? hbits : 12, dpad,
+                                       0, 0, 0);
   DG_CUDA(cudaFuncSetAttribute(sk, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)std::max(limit.total * 4, Ly.total * 4)));
   int sblocks = 0;

@@ -845,6 +845,7 @@ DgStatus dg_search_batch(DgIndex *idx, const DgSearchParams *p, const float *que
     DG_CUDA(cudaMemsetAsync(aa.counter, 0, 4, ss));
     const SearchPlan P =
         plan_search(idx, trav, lcap, filt, need, search_k, reranked, sched, nq, a.out_stats != nullptr);
+    if (idx->forcing) idx->last_cta = P.cta;
     aa.limit_smem = P.limit_smem;
     aa.hbits = P.hbits;
     aa.hB = P.hB;
@@ -1013,8 +1014,13 @@ DgStatus dg_index_autotune(DgIndex *idx, const DgSearchParams *p, const float *q
     c.occ_pct = pct;
     result = consider(c, nullptr);
   }
+  bool reg_list = false;  // (a CTA per query has no such choice: the times would differ by chance)
+  {
+    std::lock_guard<std::mutex> lk(idx->mu);
+    reg_list = idx->last_cta == 0;
+  }
   for (uint32_t w : {2u, 1u}) {
-    if (result != DG_OK || !have) break;
+    if (result != DG_OK || !have || !reg_list) break;
     DgIndex::Schedule c = best;
     c.wpb = w;
     result = consider(c, nullptr);

@@ -54,6 +54,7 @@ struct DgIndex {
   bool forcing = false;   // the autotuner pins `force` while it times a candidate
   Schedule force{};
   uint32_t last_key = 0;  // key of the last search run while forcing
+  uint32_t last_cta = 0;  // its warps per query (0: the register-list kernel)
   Schedule last_tuned{};  // the schedule the last dg_index_autotune chose
   float *pivots = nullptr;  // [npiv][dpad] rows spread over the ids (query ordering)
   uint32_t npiv = 0;

@@ -514,9 +514,9 @@ static uint32_t traversal_row_bytes(const DgIndex *idx, int trav) {
 // Measured (us per call, 300k x 128, 8 / 4 / 2 / 1 warps): FP32, beam 100, 256
 // queries 785 / 823 / 951 / 1221, 740 queries 1445 / 958 / 1063 / 1332, 1200
 // queries 2168 / 1251 / 1095 / 1344, 6000 queries 9008 / 4413 / 3003 / 2459;
-// BF16 with filters, 740 queries 5261 / 3041 / 2765 / 3073 (an expansion finds
-// few new neighbours there: 4 warps never win), 3000 queries - / 8931 / 5221 /
-// 4043.  Short rows skip the 2-warp step (int8, beam 100: 1470 queries 1049 us
+// BF16 with filters and lists of 256, 740 queries 5261 / 3041 / 2765 / 3073 (an
+// expansion finds few new neighbours there, so 4 warps are left out with
+// filters; longer lists were not measured), 3000 queries - / 8931 / 5221 / 4043.  Short rows skip the 2-warp step (int8, beam 100: 1470 queries 1049 us
 // with 2 warps, 1500 queries 837 with 1).  Where a query's state leaves room
 // for few queries per SM, warps are added instead: PQ tables of 16 KB (8
 // queries), 5000 queries 7365 / 4028 / 3648 / 4430 (then 3270 with 2 warps and
@@ -832,7 +832,6 @@ DgStatus dg_search_batch(DgIndex *idx, const DgSearchParams *p, const float *que
   int lpr = 1;
   if (trav == TRAV_F32) lpr = 8;
   else if (trav == TRAV_BF16 || trav == TRAV_F16) lpr = lanes_per_row(idx->dpad / 8);
-  else if (trav == TRAV_INT8) lpr = lanes_per_row(idx->code_stride / 16);
   auto launch = [&](const SearchArgs &a0, cudaStream_t ss) -> DgStatus {
     LaunchInfo info;
     SearchArgs aa = a0;
@@ -1278,7 +1277,6 @@ extern "C" DgStatus dg_search_batch_static(DgIndex *idx, const DgSearchParams *p
   int lpr = 1;
   if (trav == TRAV_F32) lpr = 8;
   else if (trav == TRAV_BF16 || trav == TRAV_F16) lpr = lanes_per_row(idx->dpad / 8);
-  else if (trav == TRAV_INT8) lpr = lanes_per_row(idx->code_stride / 16);
   const SearchPlan P = plan_search(idx, trav, lcap, filt, need, search_k, reranked, sched, nq, false);
   a.limit_smem = P.limit_smem;
   a.hbits = P.hbits;

@@ -29,7 +29,6 @@ DgStatus cuda_fail(cudaError_t e, const char *what) {
 // geometry of the gather kernels then divides the row exactly.
 uint32_t dpad_of(uint32_t d) { return (d + 31u) & ~31u; }
 
-// Copies n host rows of d floats into device rows of dpad floats (zero padded).
 // Pinned staging of large uploads from pageable memory: kUpThreads threads copy
 // pieces of kUpPiece bytes into page-locked buffers (two each) and send them
 // from there, so that the host copies run in parallel and overlap the
@@ -64,7 +63,8 @@ __global__ void k_pad_rows(const float *__restrict__ src, uint64_t n, uint32_t d
 }
 
 // Rows i of `host` (or rows[i], when given), d floats each, to dev with rows
-// dpad floats apart (padding zero).  The source is read before this returns.
+// dpad floats apart (padding zero).  A pageable source has been read when this
+// returns; one that the caller page-locked is read in stream order.
 DgStatus upload_rows_f32(const float *host, uint64_t n, uint32_t d, uint32_t dpad, float *dev, cudaStream_t st,
                          const uint64_t *rows) {
   const size_t row = (size_t)d * sizeof(float);

@@ -9,8 +9,8 @@
 // distance, so the gathers of one expansion are all in flight at once, and all
 // threads merge the surviving keys into the list.  Results are those of
 // search_one_reg: the same distances (same summation order per row), the same
-// L smallest (distance, id) pairs after every expansion, the same visited
-// table contents (so the same counts) and the same stopping rules.
+// L smallest (distance, id) pairs after every expansion, the same stopping
+// rules and, at one size of the visited table, the same counts.
 //
 // What bounds it is the chain of one expansion, not bandwidth (cycles on one
 // 8-warp CTA of the 100k x 128 FP32 search, beam 128: neighbour list and visited
@@ -498,6 +498,9 @@ __device__ inline void search_cta(const SearchArgs &a, uint32_t q, uint8_t *sm, 
   }
 }
 
+// 20 warps per SM leave 96 registers (8 warps per query: 128).  They are not
+// enough for every form: per thread, BF16 rows with a filter spill 128-264 bytes
+// at 1 to 4 warps, without one 24-128; int8 codes 48-76 and 116-176.
 template <int NW, int TRAV, int MET, int LPR, bool TC, bool FILT>
 __global__ void __launch_bounds__(32 * NW, NW == 8 ? 2 : 20 / NW) beam_search_cta_kernel(SearchArgs a, WarpLayout Ly) {
   extern __shared__ __align__(16) uint8_t smem[];

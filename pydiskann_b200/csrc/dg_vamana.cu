@@ -118,7 +118,8 @@ static BuildLayout build_layout(uint32_t Lb, uint32_t R, uint32_t hbits, uint32_
 // One warp per node: its current neighbours with their distances, then three
 // greedy searches, each on a list merged in place (cta_merge, one warp).
 // 25k nodes x 128, R = 64, beam 128: 24 ms per pass with a second copy of the
-// list, entry-by-entry merges and FMA distances.
+// list, entry-by-entry merges and FMA distances.  Five CTAs per SM leave 96
+// registers, of which FMA distances of FP32 rows spill 144-224 bytes.
 template <int ELEM, int MET, int LPR, bool TC>
 __global__ void __launch_bounds__(128, 5) k_build_search(BuildArgs a, BuildLayout Ly) {
   extern __shared__ __align__(16) uint8_t smem[];

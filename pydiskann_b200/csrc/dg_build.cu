@@ -787,11 +787,12 @@ static DgStatus knn_tiled(const float *v, uint64_t n, uint32_t dim, uint32_t dpa
 // fill the GPU that way (ms, one list / tiles; 10k queries x 100k rows: 8-d, k = 10
 // 10.0 / 10.2, k = 100 15.6 / 31.4; 32-d, k = 32 24.8 / 19.4, k = 100 28.1 / 33.4;
 // 128-d, k = 128 86 / 53; 10k rows: 32-d, k = 10 3.3 / 3.5, k = 100 4.9 / 10.7; 1000
-// queries x 100k rows: 8-d, k = 100 6.9 / 6.8, 32-d 10.3 / 7.7).  Lists above
-// kKnnTileK do not fit a tile CTA; above 1024 coordinates tiles always win.
+// queries x 100k rows: 8-d, k = 128 6.7 / 7.4, 16-d 7.8 / 7.4, 32-d 11.0 / 8.3; 500
+// queries: 8-d 6.6 / 4.6).  Lists above kKnnTileK do not fit a tile CTA; above
+// 1024 coordinates tiles always win.
 static bool knn_by_tiles(uint64_t n, uint32_t dim, uint32_t nq, uint32_t k) {
   if (k > (uint32_t)kKnnTileK) return false;
-  return nq <= 1024 || dim > 1024 || 200.0 * k <= dim * std::sqrt((double)n);
+  return nq <= (dim < 16 ? 512u : 1024u) || dim > 1024 || 200.0 * k <= dim * std::sqrt((double)n);
 }
 
 // ------------------------------------------------------------ PQ training

@@ -8,7 +8,8 @@ from pydiskann_b200 import synth
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("n,d,nq,k", [(2000, 8, 1024, 40), (2000, 8, 1025, 40), (2500, 64, 1100, 16), (2500, 64, 1100, 17),
+@pytest.mark.parametrize("n,d,nq,k", [(2000, 8, 512, 40), (2000, 8, 513, 40), (2000, 16, 1024, 40),
+                                      (2000, 8, 1024, 40), (2000, 8, 1025, 40), (2500, 64, 1100, 16), (2500, 64, 1100, 17),
                                       (70, 3, 1300, 70), (1, 8, 1100, 1), (90, 1025, 1030, 20)])
 @pytest.mark.parametrize("metric", ["l2", "euclidean"])
 def test_exact_knn_routes(oracle, n, d, nq, k, metric):
